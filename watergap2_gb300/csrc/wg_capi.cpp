@@ -642,12 +642,13 @@ wg_status state_io(wg_ctx *ctx, const wg_state_view *v, int member, bool to_devi
                              : copy_state(ctx, ctx->sf, v, member, to_device);
 }
 
-void fill_fastmath_tables(double e2[64], double lf[129], double inv[129]) {
-  for (int j = 0; j < 64; ++j) e2[j] = exp2((double)j / 64.0);
-  for (int j = 0; j <= 128; ++j) {
-    const double F = 1.0 + j / 128.0;
-    lf[j] = log(F);
-    inv[j] = 1.0 / F;
+// Tables of wg_fastmath.cuh: 2^(j/256) and, for c_j the first multiple of 2^-31 not
+// below 1/(1 + j/256), log2(1/c_j), both in units of 2^-63.
+void fill_fastmath_tables(unsigned long long e2[256], ulonglong2 l2[256]) {
+  for (int j = 0; j < 256; ++j) {
+    e2[j] = (unsigned long long)rintl(ldexpl(exp2l(j / 256.0L), 63));
+    l2[j].y = ((1ull << 39) + 255 + j) / (256 + j);
+    l2[j].x = (unsigned long long)rintl(ldexpl(31.0L - log2l((long double)l2[j].y), 63));
   }
 }
 
@@ -1031,9 +1032,10 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     return st;
   }
   {
-    double e2[64], lf[129], inv[129];
-    fill_fastmath_tables(e2, lf, inv);
-    st = cuda_fail(ctx.get(), upload_fastmath_tables(e2, lf, inv), "fastmath tables");
+    unsigned long long e2[256];
+    ulonglong2 l2[256];
+    fill_fastmath_tables(e2, l2);
+    st = cuda_fail(ctx.get(), upload_fastmath_tables(e2, l2), "fastmath tables");
     if (st != WG_OK) return st;
   }
 
@@ -1455,9 +1457,10 @@ wg_status wg_math_eval(int32_t device, int32_t fn, const double *x, const double
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) return WG_ERR_DEVICE;
   if (cudaSetDevice(device) != cudaSuccess) return WG_ERR_DEVICE;
-  double e2[64], lf[129], inv[129];
-  fill_fastmath_tables(e2, lf, inv);
-  cudaError_t e = upload_fastmath_tables(e2, lf, inv);
+  unsigned long long e2[256];
+  ulonglong2 l2[256];
+  fill_fastmath_tables(e2, l2);
+  cudaError_t e = upload_fastmath_tables(e2, l2);
   const size_t bytes = (size_t)std::max<int64_t>(n, 1) * sizeof(double);
   double *d = nullptr;
   if (e == cudaSuccess) e = cudaMalloc((void **)&d, 3 * bytes);

@@ -783,10 +783,9 @@ cudaError_t launch_math_eval(int fn, const double *x, const double *y, double *o
   return cudaGetLastError();
 }
 
-cudaError_t upload_fastmath_tables(const double exp2_tab[64], const double logF_tab[129], const double invF_tab[129]) {
-  cudaError_t e = cudaMemcpyToSymbol(fm::g_exp2_tab, exp2_tab, 64 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(fm::g_logF_tab, logF_tab, 129 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(fm::g_invF_tab, invF_tab, 129 * sizeof(double));
+cudaError_t upload_fastmath_tables(const unsigned long long exp2_tab[256], const ulonglong2 log2_tab[256]) {
+  cudaError_t e = cudaMemcpyToSymbol(fm::g_exp2_tab, exp2_tab, 256 * sizeof(exp2_tab[0]));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(fm::g_log2_tab, log2_tab, 256 * sizeof(log2_tab[0]));
   return e;
 }
 
@@ -836,11 +835,15 @@ static const void *pipeline_fn(bool fused, bool ens, bool vaw, bool wt = false, 
                                bool vo = false, bool ro = false) {
   if (gl && (ens || wt || !wu || !std::is_same<R, double>::value)) return nullptr;   // GLWD units: FP64, one member
   if (vo || ro) {   // the output grids: FP64, one member
-    if (ens || !std::is_same<R, double>::value) return nullptr;
-    if (wt) return (wu || ro) ? nullptr : pipeline_fn_x<R, 9>(fused, vaw);   // the vertical balance's with the water temperature
-    if (gl) return pipeline_fn_x<R, 30>(fused, vaw);   // water use over GLWD units: all outputs in one variant
-    if (wu) return pipeline_fn_x<R, 26>(fused, vaw);   // with water use: all outputs in one variant
-    return ro ? pipeline_fn_x<R, 24>(fused, vaw) : pipeline_fn_x<R, 8>(fused, vaw);
+    if constexpr (std::is_same<R, double>::value) {
+      if (ens) return nullptr;
+      if (wt) return (wu || ro) ? nullptr : pipeline_fn_x<R, 9>(fused, vaw);   // the vertical balance's with the water temperature
+      if (gl) return pipeline_fn_x<R, 30>(fused, vaw);   // water use over GLWD units: all outputs in one variant
+      if (wu) return pipeline_fn_x<R, 26>(fused, vaw);   // with water use: all outputs in one variant
+      return ro ? pipeline_fn_x<R, 24>(fused, vaw) : pipeline_fn_x<R, 8>(fused, vaw);
+    } else {
+      return nullptr;
+    }
   }
   if (ens) return wt ? nullptr
                      : (wu ? (const void *)k_pipeline<R, true, true, false, 2> : (const void *)k_pipeline<R, true, true, false, 0>);

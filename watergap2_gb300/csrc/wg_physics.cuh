@@ -36,6 +36,7 @@ __device__ __forceinline__ int month_of(int doy) {
 template <class R> struct M;
 template <> struct M<double> {
   static __device__ __forceinline__ double exp(double x) { return fm::exp(x); }
+  static __device__ __forceinline__ double exp_neg(double x) { return fm::exp_neg(x); }   // exp(-x), x >= 0
   static __device__ __forceinline__ double pow(double x, double y) { return fm::pow(x, y); }
   static __device__ __forceinline__ double rcp(double x) { return fm::rcp_pos(x); }   // x normal, nonzero
   static __device__ __forceinline__ double fabs_(double x) { return fabs(x); }
@@ -44,6 +45,7 @@ template <> struct M<double> {
 };
 template <> struct M<float> {
   static __device__ __forceinline__ float exp(float x) { return expf(x); }
+  static __device__ __forceinline__ float exp_neg(float x) { return expf(-x); }
   static __device__ __forceinline__ float pow(float x, float y) { return (x > 0.f) ? powf(x, y) : 0.f; }
   static __device__ __forceinline__ float rcp(float x) { return 1.0f / x; }
   static __device__ __forceinline__ float fabs_(float x) { return fabsf(x); }
@@ -1113,7 +1115,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
   const R velocity = (c.velo_opt == 0) ? c.default_velocity : river_velocity<R>(c, s, inflow, S0);
   rt.velocity = velocity;
   const R K = velocity * c.inv_len[s];
-  const R eK = m::exp(-K);
+  const R eK = m::exp_neg(K);
   const R omeK = m::one_m_exp_neg(K, eK);
   R S, transported;
   const R remRiver0 = remainingUse;
