@@ -379,9 +379,13 @@ WarpLayout default_layout(wg_ctx *ctx) {
                                          : pipeline_max_blocks<float>(false, false, wpb * 32);
   if (fits < blocks || fits_r < blocks) return lay;
   // vertical-balance warps: fill the block to 20 warps (five per sub-partition at
-  // the 96 registers that kernel is built for), if at least two fit
-  const int va = 20 - wpb;
-  if (va >= 2 && pipeline_max_blocks<double>(true, false, (wpb + va) * 32, true) >= blocks) lay.va_warps = va;
+  // the 96 registers that kernel is built for), if at least two fit, but no more
+  // than it takes for every block to have its share: beyond that the first blocks
+  // to ask take several warps' work, their routing warps fall behind on the FP64
+  // pipe, and every block waits for them at the step barrier (4,096 cells, one
+  // year: 17 warps per block 9.4 ms, 2 warps 5.0 ms)
+  const int room = 20 - wpb, va = std::min(room, (int)((W + blocks - 1) / blocks));
+  if (room >= 2 && pipeline_max_blocks<double>(true, false, (wpb + va) * 32, true) >= blocks) lay.va_warps = va;
   // the idle warp: the last warp of the sub-partition that has the fewest warps
   // (of those that have any: a block of fewer than four warps leaves some empty)
   int cnt[4] = {0, 0, 0, 0};
