@@ -1734,10 +1734,11 @@ wg_status wg_step_routing(wg_ctx *ctx, int32_t doy, int32_t oday) {
 // call ends with the vertical state exactly at step t_e either way.
 template <class R>
 static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevStateT<R> &s, const DevVertT<R> &v,
-                                const DevRingT<R> &ring, int doy0, int fday0, int oday0, int ndays, int t_b,
+                                DevRingT<R> ring, int kd, int doy0, int fday0, int oday0, int ndays, int t_b,
                                 int t_e) {
+  ring.days_per_step = kd;
   const bool ov = ctx->overlap();
-  const int chunk = ctx->eff_chunk();
+  const int chunk = ctx->eff_chunk(kd);
   if (ctx->ens_overlap && ctx->members > 1 && ctx->va_stream) {
     // the next chunk's vertical balance on the second stream, beside this chunk's
     // wavefront launch: the vertical balance of chunk k+1 writes ring slots that
@@ -1805,13 +1806,13 @@ extern "C" {
 
 }  // extern "C"
 
-// steps [t_begin, t_end) of a run whose station and monthly outputs start at slot oday0
-static wg_status run_steps_at(wg_ctx *ctx, int doy0, int fday0, int oday0, int ndays, int t_begin, int t_end) {
+// steps [t_begin, t_end) of kd days of a run whose station and monthly outputs start at slot oday0
+static wg_status run_steps_at(wg_ctx *ctx, int kd, int doy0, int fday0, int oday0, int ndays, int t_begin, int t_end) {
   cudaSetDevice(ctx->device);
   join_uploads(ctx);
   return ctx->precision == 0
-             ? run_steps_impl(ctx, ctx->cd, ctx->sd, ctx->vd, ctx->rd, doy0, fday0, oday0, ndays, t_begin, t_end)
-             : run_steps_impl(ctx, ctx->cf, ctx->sf, ctx->vf, ctx->rf, doy0, fday0, oday0, ndays, t_begin, t_end);
+             ? run_steps_impl(ctx, ctx->cd, ctx->sd, ctx->vd, ctx->rd, kd, doy0, fday0, oday0, ndays, t_begin, t_end)
+             : run_steps_impl(ctx, ctx->cf, ctx->sf, ctx->vf, ctx->rf, kd, doy0, fday0, oday0, ndays, t_begin, t_end);
 }
 
 static wg_status vertical_now(wg_ctx *ctx, int doy, int fday) {
@@ -1852,7 +1853,8 @@ wg_status flush_deferred(wg_ctx *ctx) {
   if (q.ndays > 0) {
     const int nd = q.ndays;
     q.ndays = 0;
-    st = run_steps_at(ctx, q.doy0, q.fday0, q.oday0, nd, 0, ctx->total_steps(nd));
+    const int kd = ctx->run_days_per_step(nd);
+    st = run_steps_at(ctx, kd, q.doy0, q.fday0, q.oday0, nd, 0, ctx->total_steps(nd, kd));
     if (st == WG_OK) ctx->last_vertical_fday = q.fday0 + nd - 1;
   }
   if (st == WG_OK && q.vpending) {
@@ -1878,14 +1880,16 @@ wg_status wg_run_steps(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t ndays, 
   if (t_begin < 0 || t_end > total || t_begin > t_end) return WG_ERR_INVALID;
   WG_FLUSH(ctx);
   if (t_begin == t_end) return WG_OK;
-  return run_steps_at(ctx, doy0, fday0, fday0, ndays, t_begin, t_end);
+  return run_steps_at(ctx, ctx->days_per_step, doy0, fday0, fday0, ndays, t_begin, t_end);
 }
 
 int32_t wg_run_num_steps(const wg_ctx *ctx, int32_t ndays) { return ctx ? ctx->total_steps(ndays) : 0; }
 
 wg_status wg_run_days(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t ndays) {
-  if (!ctx) return WG_ERR_INVALID;
-  return wg_run_steps(ctx, doy0, fday0, ndays, 0, ctx->total_steps(ndays));
+  if (!ctx || doy0 < 1 || doy0 > 365 || fday0 < 0 || ndays <= 0 || fday0 + ndays > ctx->max_days) return WG_ERR_INVALID;
+  WG_FLUSH(ctx);
+  const int kd = ctx->run_days_per_step(ndays);
+  return run_steps_at(ctx, kd, doy0, fday0, fday0, ndays, 0, ctx->total_steps(ndays, kd));
 }
 
 wg_status wg_synchronize(wg_ctx *ctx) {

@@ -175,23 +175,46 @@ struct wg_ctx {
   }
   size_t nstate() const { return (size_t)n * members; }
   int ring_days() const { return precision == 0 ? rd.ring_days : rf.ring_days; }
-  // longest chunk of wavefront steps one launch pair may run: its days fit the ring
-  int max_chunk() const { return ring_days() / days_per_step; }
+  // longest chunk of wavefront steps (of kd days) one launch pair may run: its days fit the ring
+  int max_chunk(int kd) const { return ring_days() / kd; }
   // the wavefront launches carry vertical-balance warps for the next chunk
   bool overlap() const { return layout.va_warps > 0 && layout.idle_warp >= 0 && threads == layout.threads; }
   // longest chunk: with the overlap the ring holds this chunk's and the next one's days
-  int chunk_cap() const { return (overlap() || ens_overlap) ? max_chunk() / 2 : max_chunk(); }
-  // steps per launch: the set chunk length if it fits, else about 16 days with
-  // the overlap (the first chunk of each call runs its vertical balance alone)
-  // or the ring
-  int eff_chunk() const {
-    if (chunk_steps > 0 && chunk_steps <= chunk_cap()) return chunk_steps;
-    return overlap() ? std::min((16 + days_per_step - 1) / days_per_step, chunk_cap()) : chunk_cap();
+  int chunk_cap(int kd) const { return (overlap() || ens_overlap) ? max_chunk(kd) / 2 : max_chunk(kd); }
+  int chunk_cap() const { return chunk_cap(days_per_step); }
+  // steps (of kd days) per launch: the set chunk length if it fits (as many days
+  // with shorter steps), else about 16 days with the overlap (the first chunk of
+  // each call runs its vertical balance alone) or the ring
+  int eff_chunk(int kd) const {
+    if (chunk_steps > 0 && chunk_steps <= chunk_cap()) return std::min(chunk_steps * days_per_step / kd, chunk_cap(kd));
+    return overlap() ? std::min((16 + kd - 1) / kd, chunk_cap(kd)) : chunk_cap(kd);
     // (with ens_overlap the longest chunk that fits the ring: the launches of a
     // chunk pair run side by side, so fewer, longer chunks lose less at their ends)
   }
-  // wavefront steps of a run of ndays days
-  int total_steps(int ndays) const { return (ndays + days_per_step - 1) / days_per_step + topo.nlevel - 1; }
+  int eff_chunk() const { return eff_chunk(days_per_step); }
+  // wavefront steps of a run of ndays days, kd days per step
+  int total_steps(int ndays, int kd) const { return (ndays + kd - 1) / kd + topo.nlevel - 1; }
+  int total_steps(int ndays) const { return total_steps(ndays, days_per_step); }
+  // Days per step of a run made in one call (wg_run_days, the deferred per-day
+  // calls): at most days_per_step, and fewer where the run is short against the
+  // drainage depth.  A step takes the time of one cell's days, one after the other
+  // (t each), and a fixed part (its barrier and the loads it starts with: fixed x
+  // t), so a run costs (ceil(D / kd) + levels - 1) (fixed + kd) t beside its
+  // throughput: with kd days per step the fill and drain of levels - 1 steps last
+  // kd days each.  fixed was measured from runs at 1, 2, 3 and 5 days per step:
+  // 0.25 for one member (65,000 to 550,000 cells, FP64 and FP32), 6 for ensembles,
+  // whose steps start with more loads and whose days overlap across members.
+  // Global grid, one year (198 levels), 1 / 2 / 5 days per step: 18.6 / 21.4 /
+  // 30.6 ms, with water temperature, half a year: 22.0 / 30.2 / 51.2 ms, 550,000
+  // cells in FP32, 90 days: 11.0 / 13.3 / 21.6 ms, 64 FP32 members, 90 days: 33.7
+  // / 31.3 / 36.7 ms (this rule: 1, 1, 1 and 2).  Results do not depend on it.
+  int run_days_per_step(int ndays) const {
+    const double fixed = members > 1 ? 6.0 : 0.25;
+    int best = 1;
+    for (int kd = 2; kd <= days_per_step; ++kd)
+      if (total_steps(ndays, kd) * (fixed + kd) < total_steps(ndays, best) * (fixed + best)) best = kd;
+    return best;
+  }
   void release_tools();   // snapshot and graph (wg_tune.cpp)
 };
 
