@@ -612,7 +612,8 @@ wg_status wg_measure_fp64_peak(int32_t device, double *tflops);
 wg_status wg_math_eval(int32_t device, int32_t fn, const double *x, const double *y, int64_t n, double *out);
 
 /* Information: number of drainage levels (longest flow path + 1), kernel
- * launches issued so far, and the last CUDA error string. */
+ * launches issued so far (the passes over the forcing that prepare a run are not
+ * counted), and the last CUDA error string. */
 int32_t wg_num_levels(const wg_ctx *ctx);
 int64_t wg_launch_count(const wg_ctx *ctx);
 /* wg_last_error(NULL): why the calling thread's last wg_create failed. */

@@ -301,7 +301,7 @@ struct HostConsts {
   // one vector per DevCellsT field of type R
 #define WG_RFIELDS(X)                                                                                            \
   X(cfa) X(inv_cfa) X(mprec) X(alpha) X(pet_mxdy) X(mnetrad) X(mcwh) X(t_snowfz) X(t_snowmt) X(pcritgwa) X(gamma) \
-  X(albedo) X(albedo_snow) X(ddf_m) X(lai_min) X(lai_max) X(smax) X(inv_smax) X(fg) X(rgmax) X(built_up)         \
+  X(albedo) X(albedo_snow) X(ddf_m) X(lai_min) X(lai_max) X(lai_s30) X(smax) X(inv_smax) X(fg) X(rgmax) X(built_up)         \
   X(t_gradnt) X(elev0) X(contfreq) X(area) X(area_f) X(gw_e) X(gw_ik) X(gw_ome) X(sw_k) X(sw_e) X(sw_ik)        \
   X(sw_ome) X(evx)                                                                                               \
   X(a6) X(ll100) X(maxs_ll) X(inv_maxs_ll) X(lw100) X(maxs_lw) X(inv_maxs_lw) X(la6) X(maxs_gl) X(inv_maxs_gl)  \
@@ -313,16 +313,16 @@ struct HostConsts {
   std::vector<double> band_dt;   // [ncell][nband]
   std::vector<double> ext, inv_s0;
   std::vector<double> statcorr;  // G_statCorrFact (P_CFS) with statcorrOpt = 1, else empty
-  std::vector<float> snow_thr;   // [ncell][nband] FP32 paths' snowfall thresholds (snowfall_threshold)
-  std::vector<double> t_gradnt64, t_snowfz64;
+  std::vector<float> snow_thr, melt_thr;   // [ncell][nband] snowfall and melt thresholds (snowfall_threshold)
   int nrow = 0;
 };
 
 // The largest float temperature t at which a band gets snowfall as the FP64 path
 // decides it: ((double)t - band_dt) <= t_snowfz (daily.cpp:982), band_dt =
-// (elev_b - elev_0) * P_T_GRADNT in FP64.  The test is monotone in t, so the FP32
-// paths compare their float temperature with this value and take the same
-// decision for every input.
+// (elev_b - elev_0) * P_T_GRADNT in FP64.  The test is monotone in t, so the float
+// temperature is compared with this value and the decision is the same for every
+// input.  With P_T_SNOWMT in the place of t_snowfz: the largest float temperature
+// at which the band does not melt.
 float snowfall_threshold(double band_dt, double t_snowfz) {
   auto snow = [&](float t) { return ((double)t - band_dt) <= t_snowfz; };
   float t = (float)(t_snowfz + band_dt);
@@ -492,10 +492,11 @@ wg_status upload_cells(wg_ctx *ctx, const HostConsts &h, DevCellsT<R> &c, double
   WG_RFIELDS(X)
 #undef X
   c.band_dt = upload_raw<R>(ctx, bands_to_slots<double>(ctx, h.band_dt.data(), ctx->nband), st);
-  c.snow_thr = nullptr;
-  c.thr64 = nullptr;
-  if (sizeof(R) == 4) {   // the FP32 paths' snowfall decisions (vertical_cell)
-    c.snow_thr = upload_raw<float>(ctx, bands_to_slots<float>(ctx, h.snow_thr.data(), ctx->nband), st);
+  c.snow_thr = upload_raw<float>(ctx, bands_to_slots<float>(ctx, h.snow_thr.data(), ctx->nband), st);
+  c.melt_thr = nullptr;
+  if (sizeof(R) == 8) {
+    c.melt_thr = upload_raw<float>(ctx, bands_to_slots<float>(ctx, h.melt_thr.data(), ctx->nband), st);
+  } else {
     // the arid recharge rule dailyPrec <= P_PCRITGWA (daily.cpp:1172) on a float
     // precipitation: against the largest float not above the FP64 threshold it
     // takes the FP64 path's decision for every input
@@ -506,13 +507,6 @@ wg_status upload_cells(wg_ctx *ctx, const HostConsts &h, DevCellsT<R> &c, double
       pc[i] = f;
     }
     c.pcritgwa = (const R *)upload_slots<float>(ctx, pc, st);
-    std::vector<double> t64(2 * (size_t)ctx->n);
-    for (int sl = 0; sl < ctx->n; ++sl) {
-      const int cell = ctx->topo.cell_of_slot[sl];
-      t64[sl] = h.t_gradnt64[cell];
-      t64[(size_t)ctx->n + sl] = h.t_snowfz64[cell];
-    }
-    c.thr64 = upload_raw<double>(ctx, t64, st);
   }
   c.band_el = upload_raw<int16_t>(ctx, bands_to_slots<int16_t>(ctx, h.band_el.data(), ctx->nband), st);
   c.ext_rad = upload_raw<R>(ctx, h.ext, st);
@@ -647,13 +641,22 @@ wg_status state_io(wg_ctx *ctx, const wg_state_view *v, int member, bool to_devi
 }
 
 // Tables of wg_fastmath.cuh: 2^(j/256) and, for c_j the first multiple of 2^-31 not
-// below 1/(1 + j/256), log2(1/c_j), both in units of 2^-63.
-void fill_fastmath_tables(unsigned long long e2[256], ulonglong2 l2[256]) {
-  for (int j = 0; j < 256; ++j) {
-    e2[j] = (unsigned long long)rintl(ldexpl(exp2l(j / 256.0L), 63));
-    l2[j].y = ((1ull << 39) + 255 + j) / (256 + j);
-    l2[j].x = (unsigned long long)rintl(ldexpl(31.0L - log2l((long double)l2[j].y), 63));
+// below 1/(1 + j/256), log2(1/c_j), both in units of 2^-63.  Computed once per
+// process: the long double functions take 0.3 ms on a host that emulates them.
+struct FastmathTables {
+  unsigned long long e2[256];
+  ulonglong2 l2[256];
+  FastmathTables() {
+    for (int j = 0; j < 256; ++j) {
+      e2[j] = (unsigned long long)rintl(ldexpl(exp2l(j / 256.0L), 63));
+      l2[j].y = ((1ull << 39) + 255 + j) / (256 + j);
+      l2[j].x = (unsigned long long)rintl(ldexpl(31.0L - log2l((long double)l2[j].y), 63));
+    }
   }
+};
+cudaError_t upload_fastmath() {
+  static const FastmathTables t;
+  return upload_fastmath_tables(t.e2, t.l2);
 }
 
 }  // namespace
@@ -1036,10 +1039,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     return st;
   }
   {
-    unsigned long long e2[256];
-    ulonglong2 l2[256];
-    fill_fastmath_tables(e2, l2);
-    st = cuda_fail(ctx.get(), upload_fastmath_tables(e2, l2), "fastmath tables");
+    st = cuda_fail(ctx.get(), upload_fastmath(), "fastmath tables");
     if (st != WG_OK) return st;
   }
 
@@ -1061,8 +1061,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
   h.band_dt.resize((size_t)n * B);
   h.band_el.resize((size_t)n * B);
   h.snow_thr.resize((size_t)n * B);
-  h.t_gradnt64.resize(n);
-  h.t_snowfz64.resize(n);
+  h.melt_thr.resize((size_t)n * B);
   std::vector<double> lats;
   for (int i = 0; i < n; ++i) {
     const int lct = r->lct[i];
@@ -1086,6 +1085,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     const float lmin = r->lct_lai_a[lct - 1] + r->lct_lai_b[lct - 1] * r->lai_max[i];   // lai.cpp:154 (float)
     h.lai_min[i] = lmin;
     h.lai_max[i] = r->lai_max[i];
+    h.lai_s30[i] = ((double)r->lai_max[i] - (double)lmin) / 30.0;
     {   // the output grids' constants: Kc (lai.cpp:295-306, LAImin in float as there),
         // the first year's freshwater share (routing.cpp:1213), the global-lake and
         // reservoir shares, G_loc_lake / 100
@@ -1126,9 +1126,8 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
       h.band_dt[(size_t)i * B + b] = (el[b + 1] - el[0]) * P(T_GRADNT, i);
       h.band_el[(size_t)i * B + b] = el[b + 1];
       h.snow_thr[(size_t)i * B + b] = snowfall_threshold(h.band_dt[(size_t)i * B + b], P(T_SNOWFZ, i));
+      h.melt_thr[(size_t)i * B + b] = snowfall_threshold(h.band_dt[(size_t)i * B + b], P(T_SNOWMT, i));
     }
-    h.t_gradnt64[i] = P(T_GRADNT, i);
-    h.t_snowfz64[i] = P(T_SNOWFZ, i);
     const double kg = P(GWOUTF, i);
     h.gw_e[i] = exp(-1. * kg);
     h.gw_ik[i] = 1. / kg;
@@ -1213,7 +1212,8 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t)16 << 30;
     // (ensembles: 24 GB, so that the ring holds two chunks of the stream overlap)
     const size_t ring_bytes = std::min<size_t>((size_t)(ctx->members > 1 ? 24 : 8) << 30, free_b / 8);
-    const size_t budget = opt->ring_days > 0 ? (size_t)opt->ring_days : ring_bytes / (2 * elem * N);
+    // per day: surface runoff and recharge of every state, the three PETs of every cell
+    const size_t budget = opt->ring_days > 0 ? (size_t)opt->ring_days : ring_bytes / (elem * (2 * N + 3 * (size_t)n));
     const int ring = (int)std::max<size_t>(std::max(8, 2 * ctx->days_per_step),
                                            std::min<size_t>(budget, (size_t)ctx->max_days));
     ctx->rd.days_per_step = ctx->rf.days_per_step = ctx->days_per_step;
@@ -1221,17 +1221,22 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
       ctx->rd.ring_days = ring;
       ctx->rd.rs = ctx->alloc<double>((size_t)ring * N);
       ctx->rd.gwr = ctx->alloc<double>((size_t)ring * N);
-      if (!ctx->rd.gwr) return WG_ERR_NOMEM;
-      if (opt->water_temp) {   // the river's open-water terms of the cells run ahead
+      ctx->rd.pet = ctx->alloc<double>((size_t)ring * n);
+      ctx->rd.pet_snow = ctx->alloc<double>((size_t)ring * n);
+      ctx->rd.pet_water = ctx->alloc<double>((size_t)ring * n);
+      if (!ctx->rd.rs || !ctx->rd.gwr || !ctx->rd.pet || !ctx->rd.pet_snow || !ctx->rd.pet_water) return WG_ERR_NOMEM;
+      if (opt->water_temp) {   // the river's open-water precipitation of the cells run ahead
         ctx->rd.owp = ctx->alloc<double>((size_t)ring * N);
-        ctx->rd.owpet = ctx->alloc<double>((size_t)ring * N);
-        if (!ctx->rd.owpet) return WG_ERR_NOMEM;
+        if (!ctx->rd.owp) return WG_ERR_NOMEM;
       }
     } else {
       ctx->rf.ring_days = ring;
       ctx->rf.rs = ctx->alloc<float>((size_t)ring * N);
       ctx->rf.gwr = ctx->alloc<float>((size_t)ring * N);
-      if (!ctx->rf.gwr) return WG_ERR_NOMEM;
+      ctx->rf.pet = ctx->alloc<float>((size_t)ring * n);
+      ctx->rf.pet_snow = ctx->alloc<float>((size_t)ring * n);
+      ctx->rf.pet_water = ctx->alloc<float>((size_t)ring * n);
+      if (!ctx->rf.rs || !ctx->rf.gwr || !ctx->rf.pet || !ctx->rf.pet_snow || !ctx->rf.pet_water) return WG_ERR_NOMEM;
     }
   }
   float *fb = ctx->alloc<float>((size_t)3 * ctx->max_days * n);
@@ -1461,10 +1466,7 @@ wg_status wg_math_eval(int32_t device, int32_t fn, const double *x, const double
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) return WG_ERR_DEVICE;
   if (cudaSetDevice(device) != cudaSuccess) return WG_ERR_DEVICE;
-  unsigned long long e2[256];
-  ulonglong2 l2[256];
-  fill_fastmath_tables(e2, l2);
-  cudaError_t e = upload_fastmath_tables(e2, l2);
+  cudaError_t e = upload_fastmath();
   const size_t bytes = (size_t)std::max<int64_t>(n, 1) * sizeof(double);
   double *d = nullptr;
   if (e == cudaSuccess) e = cudaMalloc((void **)&d, 3 * bytes);
@@ -1747,6 +1749,8 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
     // ends with both streams joined on the context's stream
     auto va = [&](int a, int b) {
       ctx->launches++;
+      const cudaError_t pe = launch_pet(c, ctx->forcing, ring, doy0, fday0, ndays, a, b, ctx->va_stream);
+      if (pe != cudaSuccess) return pe;
       return launch_vertical_ahead(c, s, ctx->forcing, ctx->mem, ctx->balance, ring, doy0, fday0, ndays, a, b,
                                    ctx->blocks_va, ctx->threads, ctx->va_stream, ctx->mon, oday0);
     };
@@ -1777,11 +1781,20 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
   DevVaWork vw{};
   vw.next = ctx->va_next;
   vw.nitems = (int)((ctx->nstate() + 31) / 32);
+  int pet_end = t_b;   // the ring holds the PET of the steps before pet_end
   for (int a = t_b; a < t_e; a += chunk) {
     const int b = std::min(t_e, a + chunk);
     cudaEvent_t *ev = ctx->timing ? ctx->timing_events() : nullptr;
     if (ev) cudaEventRecord(ev[0], ctx->stream);
     cudaError_t e = cudaSuccess;
+    if (pet_end < std::min(t_e, ov ? b + chunk : b)) {
+      // as many steps as the ring holds from this chunk on (a whole call where it
+      // fits); the slots it overwrites were read by the launches before
+      const int to = std::min(t_e, a + ctx->max_chunk(kd));
+      e = launch_pet(c, ctx->forcing, ring, doy0, fday0, ndays, pet_end, to, ctx->stream);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "run_steps");
+      pet_end = to;
+    }
     if (!ov || a == t_b) {
       e = launch_vertical_ahead(c, s, ctx->forcing, ctx->mem, ctx->balance, ring, doy0, fday0, ndays, a, b,
                                 ctx->blocks_fused, ctx->threads, ctx->stream, ctx->mon, oday0);

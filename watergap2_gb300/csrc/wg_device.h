@@ -56,13 +56,13 @@ struct DevCellsT {
   const int32_t *station;       // station index or -1
   // vertical balance
   const R *cfa, *inv_cfa, *mprec, *alpha, *pet_mxdy, *mnetrad, *mcwh, *t_snowfz, *t_snowmt, *pcritgwa, *gamma;
-  const R *albedo, *albedo_snow, *ddf_m, *lai_min, *lai_max, *smax, *inv_smax, *fg, *rgmax, *built_up;
+  const R *albedo, *albedo_snow, *ddf_m, *lai_min, *lai_max, *lai_s30, *smax, *inv_smax, *fg, *rgmax, *built_up;
   const R *t_gradnt, *elev0;
   const R *contfreq;            // continental share of the cell [%] (the monthly output grids)
   const R *band_dt;             // [nband][n] (elev_b - elev_0) * P_T_GRADNT
-  const float *snow_thr;        // FP32 paths: [nband][n] the largest float temperature at which the
-                                // band gets snowfall as the FP64 path decides it (null in FP64)
-  const double *thr64;          // FP32 paths: [2][n] P_T_GRADNT and P_T_SNOWFZ in FP64 (null in FP64)
+  const float *snow_thr;        // [nband][n] the largest float temperature at which the band gets
+                                // snowfall as the reference's FP64 expression decides it
+  const float *melt_thr;        // FP64: the same of the band not melting (null in FP32)
   const int16_t *band_el;       // [nband][n] band elevation [m]
   // routing
   const R *area, *area_f;       // km2, km2 * 1e-8 (mm x % -> km3)
@@ -219,7 +219,10 @@ struct DevMembers {
 template <class R>
 struct DevRingT {
   R *rs, *gwr;
-  R *owp, *owpet;          // open-water precipitation and PET (only with the water temperature, else null)
+  R *owp;                  // open-water precipitation (only with the water temperature, else null)
+  // [ring_days][n]: potential evapotranspiration of every cell's land without and
+  // with snow and of open water (k_pet), the same for all members
+  R *pet, *pet_snow, *pet_water;
   int32_t ring_days;
   int32_t days_per_step;   // days every cell advances per wavefront step (K >= 1)
 };

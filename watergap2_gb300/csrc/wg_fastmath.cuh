@@ -21,8 +21,7 @@
 // the polynomials interpolated at Chebyshev nodes (errors 2^-70 and 2^-59); the
 // reciprocal from the single-precision hardware approximation by one third-order
 // Newton step (P. Markstein, "IA-64 and Elementary Functions", 2000, ch. 8) in
-// fixed point.  The tables are filled on the host by fill_fastmath_tables()
-// (wg_capi.cpp).
+// fixed point.  The tables are filled on the host (FastmathTables, wg_capi.cpp).
 //
 // pow takes x >= 0 (x <= 0 gives 0, as the hot path's pow(0, y > 0) does).
 #pragma once
@@ -50,10 +49,9 @@ __device__ __forceinline__ u64 mul_hi(u64 a, u64 b) {
   return mul_wide(hi32(a), hi32(b)) + __umulhi(hi32(a), lo32(b)) + __umulhi(lo32(a), hi32(b));
 }
 
-// 2^(n + f), f in units of 2^-64, rounded to a double.  The polynomial is exact at
-// both ends of its interval, so that 2^f keeps its accuracy on both sides of
-// f = 0: the river's 1 - exp(-K) lives on the last bits of exp(-K).
-__device__ __forceinline__ double exp2_fixed(int n, u64 f) {
+// 2^f, f in units of 2^-64, in units of 2^-63 (at least 2^63).  The polynomial is
+// exact at both ends of its interval.
+__device__ __forceinline__ u64 exp2_mant(u64 f) {
   const u64 t = g_exp2_tab[hi32(f) >> 24];
   const u64 r = f << 8;                                      // 256 (f - j/256)
   const uint32_t rh = hi32(r);
@@ -61,7 +59,12 @@ __device__ __forceinline__ double exp2_fixed(int n, u64 f) {
   const uint32_t a3 = 0xe35846b9u + __umulhi(rh, a4);
   const u64 a2 = 0x3d7f7bff0589ull + ((u64)__umulhi(rh, a3) << 4);   // units of 2^-64
   const u64 a1 = 0xb17217f7d1cf7aull + mul_hi(r, a2);
-  const u64 u = t + mul_hi(t, mul_hi(r, a1));                // units of 2^-63, at least 2^63
+  return t + mul_hi(t, mul_hi(r, a1));
+}
+
+// 2^(n + f), f in units of 2^-64, rounded to a double
+__device__ __forceinline__ double exp2_fixed(int n, u64 f) {
+  const u64 u = exp2_mant(f);
   if ((unsigned)(n + 1021) >= 2045u) {                       // subnormal, zero or infinite
     if (n > 1023) return double_of(0x7ff0000000000000ull);
     if (n < -1022) {
@@ -188,14 +191,10 @@ __device__ __forceinline__ double pow(double x, double y) {
   return exp2_fixed((int)(n ^ s), f ^ (u64)(i64)(int)s);
 }
 
-// 1/x for finite normal x of either sign, to half an ulp and 2^-8 more: the
-// single-precision hardware reciprocal r of the leading 24 bits, lowered so that
-// e = 1 - x r is positive (below 2^-20), then r (1 + e + e^2).  The hot path calls
-// it only with divisors bounded away from zero.
-__device__ __forceinline__ double rcp_pos(double x) {
-  const u64 b = bits_of(x);
-  const u64 m = (b << 11) | 0x8000000000000000ull;           // in [1, 2), units of 2^-63
-  const uint32_t ex = (hi32(b) >> 20) & 0x7ff;
+// 1/(m 2^-63) for m in [2^63, 2^64), in units of 2^-64: the single-precision
+// hardware reciprocal r of the leading 24 bits, lowered so that e = 1 - m r is
+// positive (below 2^-20), then r (1 + e + e^2)
+__device__ __forceinline__ u64 rcp_mant(u64 m) {
   float r0;                                                  // in (0.5, 1]
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(__uint_as_float(0x3f800000u | ((hi32(m) << 1) >> 9))));
   const uint32_t rb = __float_as_uint(r0);
@@ -203,7 +202,15 @@ __device__ __forceinline__ double rcp_pos(double x) {
   const u64 e = (1ull << 63) - (mul_wide(hi32(m), r) + __umulhi(lo32(m), r));               // units of 2^-63
   const uint32_t eh = (uint32_t)(e >> 20);
   const u64 g = e + (mul_wide(eh, eh) >> 23);
-  const u64 u = ((u64)r << 32) + ((mul_wide(r, hi32(g)) + __umulhi(r, lo32(g))) << 1);      // units of 2^-64
+  return ((u64)r << 32) + ((mul_wide(r, hi32(g)) + __umulhi(r, lo32(g))) << 1);
+}
+
+// 1/x for finite normal x of either sign, to half an ulp and 2^-8 more.  The hot
+// path calls it only with divisors bounded away from zero.
+__device__ __forceinline__ double rcp_pos(double x) {
+  const u64 b = bits_of(x);
+  const uint32_t ex = (hi32(b) >> 20) & 0x7ff;
+  const u64 u = rcp_mant((b << 11) | 0x8000000000000000ull);
   const double v = double_of((u >> 11) + (((u64)((2044u - ex) << 20) << 32) | ((lo32(u) >> 10) & 1u)) |
                              (b & 0x8000000000000000ull));
   // zero, subnormal, infinite and NaN arguments give NaN, those from 2^1022 on 0

@@ -176,28 +176,67 @@ __device__ __forceinline__ void store_rstate(const DevStateT<R> &s, size_t i, co
   if (fl & F_RES) { s.res[i] = r.res; s.rf_res[i] = r.rf_res; s.k_release[i] = r.k_release; }
 }
 
-// One cell-day of the vertical balance on state index si (slot s).
+// One cell-day of the vertical balance on state index si (slot s); rad: the
+// radiation terms, for the output grids.
 template <class R>
 __device__ __forceinline__ void vertical_at(const DevCellsT<R> &c, const DevStateT<R> &st, size_t N, int s,
-                                            size_t si, int doy, R Pin, R gamma_soil, float Tf, float SWf, R laf,
-                                            R prev, VOut<R> &o, const VSink *vs = nullptr) {
+                                            size_t si, R Pin, R gamma_soil, float Tf, const Pet<R> &pet, R laf, R prev,
+                                            VOut<R> &o, const VSink *vs = nullptr, const Radiation<R> *rad = nullptr,
+                                            R ext_rad = R(0)) {
   if (c.flags[s] & F_NOCONT) {   // no vertical balance: the terms stay 0, the state as it is
     o.rs = R(0); o.gwr = R(0); o.transfer = R(0); o.owp = R(0); o.owpet = R(0);
     o.land_in = R(0); o.land_evap = R(0); o.land_leak = R(0);
     return;
   }
-  const size_t ti = (size_t)(doy - 1) * c.nrow + c.ext_row[s];
-  const R ext = c.ext_rad[ti], inv_s0 = c.inv_s0[ti];
   R canopy = st.canopy[si], soil = st.soil[si], gsnow = st.snow[si], psum = st.lai_precsum[si];
   int days = st.lai_days[si], status = st.lai_status[si];
   if (vs)   // the output grids (FP64 single member)
     vertical_cell<R, std::is_same<R, double>::value>(c, s, gamma_soil, canopy, soil, gsnow, st.snow_band + si, N,
-                                                      days, status, psum, laf, prev, Pin, Tf, SWf, ext, inv_s0, o, vs);
+                                                      days, status, psum, laf, prev, Pin, Tf, pet, o, vs, rad, ext_rad);
   else
     vertical_cell<R>(c, s, gamma_soil, canopy, soil, gsnow, st.snow_band + si, N, days, status, psum, laf, prev, Pin,
-                     Tf, SWf, ext, inv_s0, o);
+                     Tf, pet, o);
   st.canopy[si] = canopy; st.soil[si] = soil; st.snow[si] = gsnow; st.lai_precsum[si] = psum;
   st.lai_days[si] = days; st.lai_status[si] = status;
+}
+
+// The radiation terms of slot s on a day of the year.
+template <class R>
+__device__ __forceinline__ Radiation<R> radiation_at(const DevCellsT<R> &c, int s, int doy, float Tf, float SWf) {
+  const size_t ti = (size_t)(doy - 1) * c.nrow + c.ext_row[s];
+  return radiation<R>(c, s, Tf, SWf, c.ext_rad[ti], c.inv_s0[ti]);
+}
+
+template <class R>
+__device__ __forceinline__ Pet<R> ring_pet(const DevRingT<R> &ring, size_t k) {
+  return Pet<R>{ring.pet[k], ring.pet_snow[k], ring.pet_water[k]};
+}
+
+// Potential evapotranspiration of the days that the wavefront steps [t_b, t_e) will
+// route, every cell, into the ring: it depends on the forcing alone, not on the
+// state or the member, so it is taken out of the day-after-day chains of the
+// vertical balance (which two thirds of its FP64 and integer instructions then
+// leave) into a launch that runs all cell-days side by side.  A thread runs
+// kPetDays days of its slot; the ring's rows are written coalesced where a warp's
+// cells share their wavefront offset.  Bound by the integer pipe (fixed point);
+// KPET.
+constexpr int kPetDays = 8;
+template <class R>
+__global__ void __launch_bounds__(256) k_pet(DevCellsT<R> c, DevForcing f, DevRingT<R> ring, int doy0, int fday0,
+                                             int ndays, int t_b, int t_e) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= c.n || (c.active && !c.active[s]) || (c.flags[s] & F_NOCONT)) return;
+  const int kd = ring.days_per_step;
+  const long long first = (long long)kd * (t_b - c.offset[s]) + (long long)blockIdx.y * kPetDays;
+  const int d0 = (int)max(0ll, first);
+  const int d1 = (int)min(min(first + kPetDays, (long long)kd * (t_e - c.offset[s])), (long long)ndays);
+  for (int d = d0; d < d1; ++d) {
+    const size_t fo = (size_t)(fday0 + d) * c.n + s, k = (size_t)(d % ring.ring_days) * c.n + s;
+    const Pet<R> p = pet_of<R>(c, s, radiation_at<R>(c, s, (doy0 - 1 + d) % 365 + 1, f.temp[fo], f.swrad[fo]));
+    ring.pet[k] = p.land;
+    ring.pet_snow[k] = p.snow;
+    ring.pet_water[k] = p.water;
+  }
 }
 
 template <class R>
@@ -209,8 +248,9 @@ __global__ void __launch_bounds__(256) k_vertical(DevCellsT<R> c, DevStateT<R> s
   VOut<R> o;
   const R laf = st.laf[s];
   const R prev = (st.laf_started[s] == 1) ? st.laf_prev[s] : laf;   // daily.cpp:159-169
-  vertical_at<R>(c, st, (size_t)c.n, s, (size_t)s, doy, R(f.prec[fo]), c.gamma[s], f.temp[fo], f.swrad[fo], laf, prev,
-                 o);
+  const float Tf = f.temp[fo];
+  const Pet<R> pet = pet_of<R>(c, s, radiation_at<R>(c, s, doy, Tf, f.swrad[fo]));
+  vertical_at<R>(c, st, (size_t)c.n, s, (size_t)s, R(f.prec[fo]), c.gamma[s], Tf, pet, laf, prev, o);
   v.rs[s] = o.rs; v.gwr[s] = o.gwr; v.transfer[s] = o.transfer; v.owp[s] = o.owp; v.owpet[s] = o.owpet;
   v.land_in[s] = o.land_in; v.land_evap[s] = o.land_evap; v.land_leak[s] = o.land_leak;
 }
@@ -271,23 +311,23 @@ __device__ __forceinline__ void va_cell(const DevCellsT<R> &c, const DevStateT<R
   for (int d = d0; d < d1; ++d) {
     const int doy = (doy0 - 1 + d) % 365 + 1;
     const size_t fo = (size_t)(fday0 + d) * n + s;
-    const size_t ti = (size_t)(doy - 1) * c.nrow + c.ext_row[s];
+    const float Tf = f.temp[fo];
+    const Pet<R> pet = ring_pet(ring, (size_t)(d % ring.ring_days) * n + s);
     VOut<R> o;
     VSink vs;
-    if (!ENS && mon && vert_sink(*mon, oday0 + d, i, N, vs))   // the output grids (FP64 single member)
+    if (!ENS && mon && vert_sink(*mon, oday0 + d, i, N, vs)) {   // the output grids (FP64 single member)
+      const Radiation<R> rad = radiation_at<R>(c, s, doy, Tf, f.swrad[fo]);
       vertical_cell<R, std::is_same<R, double>::value>(c, s, gam, canopy, soil, gsnow, st.snow_band + i, N, days,
-                                                        status, psum, laf, laf, R(f.prec[fo]) * pf, f.temp[fo],
-                                                        f.swrad[fo], c.ext_rad[ti], c.inv_s0[ti], o, &vs);
-    else
+                                                        status, psum, laf, laf, R(f.prec[fo]) * pf, Tf, pet, o, &vs,
+                                                        &rad, c.ext_rad[(size_t)(doy - 1) * c.nrow + c.ext_row[s]]);
+    } else {
       vertical_cell<R>(c, s, gam, canopy, soil, gsnow, st.snow_band + i, N, days, status, psum, laf, laf,
-                       R(f.prec[fo]) * pf, f.temp[fo], f.swrad[fo], c.ext_rad[ti], c.inv_s0[ti], o);
+                       R(f.prec[fo]) * pf, Tf, pet, o);
+    }
     const size_t ri = (size_t)(d % ring.ring_days) * N + i;
     ring.rs[ri] = o.rs;
     ring.gwr[ri] = o.gwr;
-    if (ring.owp) {   // the water temperature's open-water terms of the river
-      ring.owp[ri] = o.owp;
-      ring.owpet[ri] = o.owpet;
-    }
+    if (ring.owp) ring.owp[ri] = o.owp;   // the river's, for the water temperature
     if (b.enabled) {
       acc_in += (double)o.land_in * land_f;
       acc_ev += (double)o.land_evap * land_f;
@@ -434,7 +474,7 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
             o.land_in = R(0); o.land_evap = R(0); o.land_leak = R(0);   // accounted ahead
             if constexpr (WT) {
               o.owp = ring.owp[ri];
-              o.owpet = ring.owpet[ri];
+              o.owpet = ring.pet_water[ri];   // one member: the same index
             }
           } else if (FUSED) {
             const size_t fo = (size_t)(fday0 + d) * n + s;
@@ -455,8 +495,16 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
               const double fll = (ll > 0. && rf > 0.) ? rf * ll : 0.;              // G_fLocLake
               vk[3 * N] = vk[4 * N] + fll * 100. + vk[5 * N];
             }
-            vertical_at<R>(c, st, N, s, si, doy, Pin, gam, f.temp[fo], f.swrad[fo], laf,
-                           started == 1 ? laf_prev : laf, o, vo ? &vs : nullptr);   // daily.cpp:159-169
+            const float Tf = f.temp[fo];
+            const Pet<R> pet = ring_pet(ring, (size_t)(d % ring.ring_days) * n + s);
+            const R prev = started == 1 ? laf_prev : laf;   // daily.cpp:159-169
+            if (VO && vo) {
+              const Radiation<R> rad = radiation_at<R>(c, s, doy, Tf, f.swrad[fo]);
+              vertical_at<R>(c, st, N, s, si, Pin, gam, Tf, pet, laf, prev, o, &vs, &rad,
+                             c.ext_rad[(size_t)(doy - 1) * c.nrow + c.ext_row[s]]);
+            } else {
+              vertical_at<R>(c, st, N, s, si, Pin, gam, Tf, pet, laf, prev, o);
+            }
           } else {
             o.rs = v.rs[s]; o.gwr = v.gwr[s]; o.transfer = v.transfer[s]; o.owp = v.owp[s]; o.owpet = v.owpet[s];
             o.land_in = v.land_in[s]; o.land_evap = v.land_evap[s]; o.land_leak = v.land_leak[s];
@@ -823,6 +871,15 @@ cudaError_t launch_vertical_ahead(const DevCellsT<R> &c, const DevStateT<R> &s, 
   return cudaGetLastError();
 }
 
+template <class R>
+cudaError_t launch_pet(const DevCellsT<R> &c, const DevForcing &f, const DevRingT<R> &ring, int doy0, int fday0,
+                       int ndays, int t_b, int t_e, cudaStream_t st) {
+  const long long days = (long long)ring.days_per_step * (t_e - t_b);
+  const dim3 grid((unsigned)((c.n + 255) / 256), (unsigned)((days + kPetDays - 1) / kPetDays));
+  k_pet<R><<<grid, 256, 0, st>>>(c, f, ring, doy0, fday0, ndays, t_b, t_e);
+  return cudaGetLastError();
+}
+
 template <class R, int X>
 static const void *pipeline_fn_x(bool fused, bool vaw) {
   return vaw ? (fused ? (const void *)k_pipeline<R, true, false, true, X> : nullptr)
@@ -947,6 +1004,8 @@ cudaError_t launch_balance_sum(const DevCellsT<R> &c, const DevStateT<R> &s, int
 #define WG_INSTANTIATE(R)                                                                                          \
   template cudaError_t launch_vertical<R>(const DevCellsT<R> &, const DevStateT<R> &, const DevVertT<R> &,        \
                                           const DevForcing &, int, int, cudaStream_t);                             \
+  template cudaError_t launch_pet<R>(const DevCellsT<R> &, const DevForcing &, const DevRingT<R> &, int, int, int,  \
+                                     int, int, cudaStream_t);                                                      \
   template int pipeline_max_blocks<R>(bool, bool, int, bool, bool, bool);                                        \
   template int vertical_ahead_max_blocks<R>(bool, int);                                                           \
   template cudaError_t launch_pipeline<R>(bool, const DevCellsT<R> &, const DevStateT<R> &, const DevVertT<R> &,  \

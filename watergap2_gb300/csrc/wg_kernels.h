@@ -47,6 +47,11 @@ cudaError_t launch_unf_forcing(const uint32_t *raw, float *dst, const int32_t *c
 template <class R>
 cudaError_t launch_vertical(const DevCellsT<R> &c, const DevStateT<R> &s, const DevVertT<R> &v, const DevForcing &f,
                             int doy, int fday, cudaStream_t st);
+// potential evapotranspiration of the days of steps [t_b, t_e) into the ring, before
+// the launches that read them
+template <class R>
+cudaError_t launch_pet(const DevCellsT<R> &c, const DevForcing &f, const DevRingT<R> &ring, int doy0, int fday0,
+                       int ndays, int t_b, int t_e, cudaStream_t st);
 template <class R>
 int pipeline_max_blocks(bool fused, bool ens, int threads, bool vaw = false, bool wt = false, bool wu = false);
 // blocks of k_vertical_ahead resident on the whole device at once (its own occupancy)

@@ -17,7 +17,10 @@
 // of these changes a result by a few ulp at most, far inside the 1e-10 bound.
 #pragma once
 #include "wg_device.h"
+#include <type_traits>
+
 #include "wg_fastmath.cuh"
+#include "wg_radiation.cuh"
 #include "wg_wtemp.cuh"
 
 namespace wg {
@@ -181,6 +184,43 @@ __device__ __forceinline__ R lai_nogrowing(int &days, int init, int &status, R l
   return lmax;
 }
 
+// Both of the above in FP64, branch-free but for integers: the lanes of a warp are in
+// different states of their leaf area, and four branches of four FP64 operations
+// each cost sixteen, one sum and one multiply-add two (s30: (lmax - lmin) / 30).
+__device__ __forceinline__ double lai_fp64(bool warm, int &days, int init, int &status, bool evergreen, bool arid,
+                                           double lmin, double lmax, double s30, double &psum, double prec) {
+  const double p = psum + prec;
+  int k = 0;   // days up from lmin (positive) or down from lmax (negative)
+  bool from_max = false;
+  if (status == 0) {
+    psum = p;
+    if (warm ? days >= init : days > init) {
+      days++;
+      if (C<double>::gt_c(p, 40.)) {
+        if (days >= init + 30) { days = init + 30; status = 1; }
+        k = days - init;
+      } else {
+        days = init;
+      }
+    } else if (warm) {
+      days++;
+    }
+  } else {
+    from_max = true;
+    if (days <= 30) {
+      days--;
+      if (warm && evergreen) status = 0;
+      if (days <= 0) { days = 0; status = 0; psum = 0.; }
+      k = days - 30;
+    } else if (warm && !(arid && C<double>::lt_c(prec, 0.5))) {
+      days = 30 + init;
+    } else {
+      days--;
+    }
+  }
+  return fma((double)k, s30, from_max ? lmax : lmin);
+}
+
 // Where one cell-day's output terms go (FP64): the sums of the day's month, field
 // k at mo[k * mos] (DevMonthly::vert; null: none), the day's values, field k at
 // dd[k * dds] (DevMonthly::dvert; null: none), and the cell's constants for Kc and
@@ -194,18 +234,81 @@ struct VSink {
   size_t vks;
 };
 
+// The radiation terms of one cell-day (daily.cpp:366-532) before the albedo, which
+// depends on the cell's snow; nothing here depends on the model's state.
+template <class R>
+struct Radiation { R solar_rad, net_lw, apet; };
+
+template <class R>
+__device__ __forceinline__ Radiation<R> radiation(const DevCellsT<R> &c, int s, float Tf, float SWf, R ext_rad, R inv_s0) {
+  typedef M<R> m;
+  typedef C<R> cmp;
+  const bool arid = (c.flags[s] & F_ARID) != 0;
+  const R a_c = arid ? R(1.35) : R(1.00), b_c = arid ? R(-0.35) : R(0.00);
+  const R T = R(Tf), alpha = c.alpha[s];
+  // the terms of the temperature alone (daily.cpp:382-387, 484-532)
+  R rlh, apt, lwt;
+  if constexpr (sizeof(R) == 4) {
+    const R inv_t2 = m::rcp(T + R(237.3));
+    const R e_s = R(0.6108) * m::exp(R(17.27) * T * inv_t2);
+    rlh = m::rcp((Tf > 0.f) ? R(2.501) - R(0.002361) * T : R(2.835));
+    apt = R(4098.) * e_s * (inv_t2 * inv_t2);
+    lwt = R(-0.02) + R(0.261) * m::exp(R(-0.000777) * T * T);
+  } else {
+    const fm::TempTerms tt = fm::temp_terms(Tf);
+    rlh = tt.rlh;
+    apt = tt.apt;
+    lwt = tt.lwt;
+  }
+  Radiation<R> o;
+  o.solar_rad = R(0.0864) * rlh * R(SWf);
+  R solar_fraction = (ext_rad == R(0)) ? R(0) : o.solar_rad * inv_s0;          // daily.cpp:430-448
+  if (cmp::gt_c(solar_fraction, R(1.))) solar_fraction = R(1.);
+  const R ff = a_c * solar_fraction + b_c;
+  if constexpr (sizeof(R) == 4) {
+    const R tK = T + R(273.2);
+    const R tK2 = tK * tK;
+    o.net_lw = (-ff * lwt * R(0.000000004903) * (tK2 * tK2)) * rlh;
+    o.apet = alpha * apt * m::rcp(apt + R(0.0016286 * 101.3) * rlh);
+  } else {
+    o.net_lw = -ff * lwt;
+    o.apet = alpha * apt;
+  }
+  return o;
+}
+
+// The day's potential evapotranspiration: of land without and with snow (the two
+// albedos), and of open water.
+template <class R>
+struct Pet { R land, snow, water; };
+
+template <class R>
+__device__ __forceinline__ Pet<R> pet_of(const DevCellsT<R> &c, int s, const Radiation<R> &r) {
+  typedef C<R> cmp;
+  auto pos = [&](R net) { return cmp::le0(net) ? R(0) : r.apet * net; };
+  const R mn = c.mnetrad[s];
+  Pet<R> p;
+  p.land = pos(mn * (r.solar_rad * (R(1.) - c.albedo[s]) + r.net_lw));
+  p.snow = pos(mn * (r.solar_rad * (R(1.) - c.albedo_snow[s]) + r.net_lw));
+  p.water = pos(r.solar_rad * R(1. - 0.08) + r.net_lw);
+  return p;
+}
+
 // dailyWaterBalanceClass::calcNewDay for one cell (daily.cpp:94-1257).
 //   c, s        : per-cell constants and the cell's slot
 //   gamma_soil  : runoff exponent (P_GAMRUN_C, times a member's factor in an ensemble)
 //   canopy ...  : the cell's state, read and written through references
 //   band        : the cell's snow bands, band[e * bstride]
 //   Pin         : precipitation (times a member's factor in an ensemble)
-//   OUT, vs     : the output grids (monthly and daily) of the cell-day
+//   pet         : the day's potential evapotranspiration
+//   OUT, vs     : the output grids (monthly and daily) of the cell-day, which take
+//                 its radiation terms rad and ext_rad too
 template <class R, bool OUT = false>
 __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R gamma_soil, R &canopy, R &soil,
                                               R &gsnow, R *band, size_t bstride, int &days, int &status, R &psum,
-                                              R landAreaFrac, R prevLAF, R Pin, float Tf, float SWf, R ext_rad,
-                                              R inv_s0, VOut<R> &o, const VSink *vs = nullptr) {
+                                              R landAreaFrac, R prevLAF, R Pin, float Tf, const Pet<R> &pet, VOut<R> &o,
+                                              const VSink *vs = nullptr, const Radiation<R> *rad = nullptr,
+                                              R ext_rad = R(0)) {
   typedef M<R> m;
   const int B = c.nband;
   const R invB = c.invB;
@@ -215,39 +318,24 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
   const R cfa = c.cfa[s];
   R dailyPrec = c.mprec[s] * Pin;                                 // daily.cpp:248
   const R T = R(Tf);
-  const R temp2 = T + R(237.3);
-  const R inv_t2 = m::rcp(temp2);
-  const R e_s = R(0.6108) * m::exp(R(17.27) * T * inv_t2);
-  const R alpha = c.alpha[s], maxDailyPET = c.pet_mxdy[s];
-  const R a_c = arid ? R(1.35) : R(1.00), b_c = arid ? R(-0.35) : R(0.00);
+  constexpr bool fp32 = sizeof(R) == 4;
+  const R maxDailyPET = c.pet_mxdy[s];
 
   // LAI state machine (lai.cpp:152-177); the temperature tests use the float input
   R dailyLai;
-  if (Tf > 8.f)
+  if constexpr (!fp32)
+    dailyLai = lai_fp64(Tf > 8.f, days, c.init_days[s], status, (flags & F_EVERGREEN) != 0, arid, c.lai_min[s],
+                        c.lai_max[s], c.lai_s30[s], psum, dailyPrec);
+  else if (Tf > 8.f)
     dailyLai = lai_growing<R>(days, c.init_days[s], status, (flags & F_EVERGREEN) != 0, arid, c.lai_min[s], c.lai_max[s],
                               psum, dailyPrec);
   else
     dailyLai = lai_nogrowing<R>(days, c.init_days[s], status, c.lai_min[s], c.lai_max[s], psum, dailyPrec);
 
   typedef C<R> cmp;
-  const R albedo = cmp::gt_c(gsnow, R(3.)) ? c.albedo_snow[s] : c.albedo[s];                 // daily.cpp:366-379
-  const R lat_heat = (Tf > 0.f) ? R(2.501) - R(0.002361) * T : R(2.835);      // daily.cpp:382-387
-  const R rlh = m::rcp(lat_heat);
-  const R solar_rad = R(0.0864) * rlh * R(SWf);
-  R solar_fraction = (ext_rad == R(0)) ? R(0) : solar_rad * inv_s0;          // daily.cpp:430-448
-  if (cmp::gt_c(solar_fraction, R(1.))) solar_fraction = R(1.);
-  const R ff = a_c * solar_fraction + b_c;
-  const R net_emissivity = R(-0.02) + R(0.261) * m::exp(R(-0.000777) * T * T);
-  const R tK = T + R(273.2);
-  const R tK2 = tK * tK;
-  const R net_lw = (-ff * net_emissivity * R(0.000000004903) * (tK2 * tK2)) * rlh;
-  const R net_rad = c.mnetrad[s] * (solar_rad * (R(1.) - albedo) + net_lw);
-  const R ow_net_rad = solar_rad * R(1. - 0.08) + net_lw;
-  const R inc_svp = R(4098.) * e_s * (inv_t2 * inv_t2);                     // daily.cpp:484-532
-  const R gamma = R(0.0016286 * 101.3) * rlh;
-  const R apet = alpha * inc_svp * m::rcp(inc_svp + gamma);
-  const R dailyPET = cmp::le0(net_rad) ? R(0) : apet * net_rad;
-  const R owPET = cmp::le0(ow_net_rad) ? R(0) : apet * ow_net_rad;
+  const bool snowy = cmp::gt_c(gsnow, R(3.));                                 // daily.cpp:366-379
+  const R dailyPET = snowy ? pet.snow : pet.land;
+  const R owPET = pet.water;
   o.owp = dailyPrec;
   o.owpet = owPET;
   // the output grids: the monthly sums (daily.cpp:1281-1386, grid_store 2) and the
@@ -264,7 +352,10 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
   [[maybe_unused]] double mw = 0.;       // landAreaFrac / contfreq
   if constexpr (OUT) {
     if (vs) {
-      const double conv = (double)lat_heat * (1.0 / 0.0864);
+      const R albedo = snowy ? c.albedo_snow[s] : c.albedo[s];
+      const R solar_rad = rad->solar_rad, net_lw = rad->net_lw;
+      const R net_rad = c.mnetrad[s] * (solar_rad * (R(1.) - albedo) + net_lw);
+      const double conv = ((Tf > 0.f) ? 2.501 - 0.002361 * (double)T : 2.835) * (1.0 / 0.0864);   // latent heat
       const double ns = (double)solar_rad * (1. - (double)albedo);
       const double cf = (double)c.contfreq[s], rcf = fm::rcp_pos(cf);
       const double lf = (double)landAreaFrac, lf100 = lf * 0.01;
@@ -318,6 +409,9 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
   // then the storages are not rescaled (x * 1 = x)
   const R ratio = !land ? R(0) : (prevLAF == landAreaFrac ? R(1) : prevLAF / landAreaFrac);
   const bool rescale = !cmp::is_one(ratio);
+  // the correction factor is 1 in most cells: its products and the storage change
+  // they weigh (the same bits: x * 1 = x, y * 0 + x * 1 = x) are left out there
+  const bool corrected = !cmp::is_one(cfa);
 
   // interception (daily.cpp:825-895)
   [[maybe_unused]] R out_maxcs = R(0);   // max_canopy_storage, 0 without leaves (daily.cpp:789, 847)
@@ -353,7 +447,7 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
       prec_to_soil = dailyPrec;
       soilPET = dailyPET;
     }
-    lsc += canopy - initialStorage;
+    if (corrected) lsc += canopy - initialStorage;
   }
   if (cmp::lt0(soilPET)) soilPET = R(0);
   if constexpr (OUT) {
@@ -374,30 +468,32 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
 
   // snow in elevation bands (daily.cpp:897-1062).  Whether a band gets snowfall
   // (temp_elev <= P_T_SNOWFZ, daily.cpp:982) decides where the day's precipitation
-  // goes; the FP32 paths take that decision as the FP64 path does, from the float
-  // temperature and a per-band float threshold prepared on the host, so that FP32
-  // rounding of temp_elev never moves a band's precipitation between snow and rain.
-  constexpr bool fp32 = sizeof(R) == 4;
+  // goes; it is monotone in the temperature, so the float temperature is compared
+  // with the largest one at which the FP64 expression says yes, prepared on the
+  // host per band: the reference's decision in both precisions, and no FP64
+  // operation for a band without snow.
   R snowChange = R(0), gs = R(0);
-  // the monthly outputs' band sums (daily.cpp:983, 998, 1032-1041): the bands with
-  // snowfall and with rain (each adds the day's precipitation above the canopy;
-  // counted on the integer pipe and multiplied once), melt, snow-covered bands
-  [[maybe_unused]] int n_snowfall = 0, n_rainfall = 0, n_cover = 0;
-  [[maybe_unused]] R out_melt = R(0);
+  // bands with snowfall and with rain (each adds the day's precipitation above the
+  // canopy; counted on the integer pipe), melt, snow-covered bands: the monthly
+  // outputs' band sums (daily.cpp:983, 998, 1032-1041) and, in FP64, effPrec, whose
+  // up to nband additions of the same precipitation become one multiplication
+  int n_rainfall = 0;
+  [[maybe_unused]] int n_snowfall = 0, n_cover = 0;
+  R out_melt = R(0);
   bool above0 = cmp::gt(R(0), c.t_snowfz[s]);   // band 0 above freezing: the soil runs (daily.cpp:1076)
-  int thresh = 0;
-  const R t_snowfz = c.t_snowfz[s], t_snowmt = c.t_snowmt[s], ddf_m = c.ddf_m[s];
+  int thresh = 0, thresh_band = 0, n_evap = 0;   // n_evap: bands that evaporate all of soilPET
+  bool any_snow = false;
+  const R t_snowmt = c.t_snowmt[s], ddf_m = c.ddf_m[s];
   for (int e = 0; e < B; ++e) {
     R sb = band[e * bstride];
-    R temp_elev = T - c.band_dt[(size_t)e * c.n + s];
-    bool snowfall = fp32 ? Tf <= c.snow_thr[(size_t)e * c.n + s] : cmp::le(temp_elev, t_snowfz);
+    bool snowfall = Tf <= c.snow_thr[(size_t)e * c.n + s];
     if (land && cmp::is_zero(sb) && !snowfall) {
       // no snow and no snowfall in this band: the steps below would keep it at
       // zero, melt nothing and pass the precipitation on -- the same bits, without
       // the band's arithmetic and store
       if (e == 0) above0 = true;
-      effPrec += prec_to_soil;
-      if constexpr (OUT) ++n_rainfall;
+      if constexpr (fp32) effPrec += prec_to_soil;
+      ++n_rainfall;
       continue;
     }
     if (!land) {
@@ -405,6 +501,8 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
       sb = R(0);
       gs = R(0);
     } else {
+      any_snow = true;
+      int tb = e;   // the band whose elevation gives the temperature
       R effBefore, melt = R(0);
       if (rescale) sb *= ratio;
       if (cmp::abs_le_c(sb, R(WG_MIN_STOR_VOL))) sb = R(0);
@@ -412,17 +510,12 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
       if (cmp::gt_c(sb, R(1000.))) {
         if (thresh == 0) {
           thresh = c.band_el[(size_t)e * c.n + s];
+          thresh_band = e;
         } else if (thresh > 0) {
-          // the remembered threshold elevation's temperature, rounded as the reference
-          // rounds it (no contraction into an FMA); the FP32 paths decide in FP64
-          temp_elev = T - (R(thresh) - c.elev0[s]) * c.t_gradnt[s];
-          if constexpr (fp32) {
-            const double te = __dsub_rn((double)Tf, __dmul_rn((double)thresh - (double)c.elev0[s], c.thr64[s]));
-            snowfall = te <= c.thr64[(size_t)c.n + s];
-          } else {
-            temp_elev = __dsub_rn(T, __dmul_rn(R(thresh) - c.elev0[s], c.t_gradnt[s]));
-            snowfall = cmp::le(temp_elev, t_snowfz);
-          }
+          // the remembered threshold elevation's temperature: that band's, by the
+          // reference's own expression (band_dt)
+          tb = thresh_band;
+          snowfall = Tf <= c.snow_thr[(size_t)tb * c.n + s];
         }
       }
       if (snowfall) {
@@ -430,15 +523,26 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
         sb += prec_to_soil;
         if (cmp::gt(sb, soilPET)) {
           sb -= soilPET;
-          snowEvapo += soilPET;
+          if constexpr (fp32) snowEvapo += soilPET;
+          else ++n_evap;
         } else {
           snowEvapo += sb;
           sb = R(0);
         }
       } else {
         effBefore = prec_to_soil;
+        ++n_rainfall;
       }
-      if (cmp::gt(temp_elev, t_snowmt) && !cmp::lt0(sb)) {
+      bool melts;
+      R temp_elev;
+      if constexpr (fp32) {
+        temp_elev = tb == e ? T - c.band_dt[(size_t)e * c.n + s] : T - (R(thresh) - c.elev0[s]) * c.t_gradnt[s];
+        melts = cmp::gt(temp_elev, t_snowmt);
+      } else {   // a cold band needs no temperature
+        melts = !(Tf <= c.melt_thr[(size_t)tb * c.n + s]);
+        if (melts) temp_elev = T - c.band_dt[(size_t)tb * c.n + s];
+      }
+      if (melts && !cmp::lt0(sb)) {
         melt = ddf_m * (temp_elev - t_snowmt);
         if (cmp::gt(melt, sb)) {
           melt = sb;
@@ -447,25 +551,35 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
           sb -= melt;
         }
       }
-      snowChange += sb - initialStorage;
+      if (corrected) snowChange += sb - initialStorage;
       if (e == 0) above0 = !snowfall;
       gs += sb;
-      effPrec += effBefore + melt;
+      if constexpr (fp32) effPrec += effBefore + melt;
+      if constexpr (OUT || !fp32) {
+        if (melts) out_melt += melt;
+      }
       if constexpr (OUT) {
         if (snowfall) ++n_snowfall;
-        else ++n_rainfall;
-        out_melt += melt;
         if (cmp::gt0(sb)) ++n_cover;
       }
     }
     band[e * bstride] = sb;
   }
   if (land) {
-    gs *= invB;
-    effPrec *= invB;
-    snowEvapo *= invB;
-    snowChange *= invB;
-    lsc += snowChange;
+    if constexpr (fp32) {
+      effPrec *= invB;
+    } else {
+      if (!cmp::is_zero(prec_to_soil)) effPrec = n_rainfall == B ? prec_to_soil : (double)n_rainfall * invB * prec_to_soil;
+      if (!cmp::is_zero(out_melt)) effPrec += out_melt * invB;
+    }
+    if (any_snow) {   // else all zero
+      gs *= invB;
+      if constexpr (!fp32) {
+        if (n_evap) snowEvapo = fma((double)n_evap, soilPET, snowEvapo);
+      }
+      snowEvapo *= invB;
+      if (corrected) lsc += snowChange * invB;
+    }
   }
   gsnow = gs;
   if constexpr (OUT) {
@@ -515,7 +629,7 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
     if (above0) {
       if (cmp::gt0(Smax)) {
         const R sat = soil * c.inv_smax[s];
-        runoff = effPrec * m::pow(sat, gamma_soil);
+        if (!cmp::is_zero(effPrec)) runoff = effPrec * m::pow(sat, gamma_soil);
         const R lim = (maxDailyPET - canopyEvapo) * sat;
         dailyAET = cmp::gt(soilPET, lim) ? lim : soilPET;
         soil += effPrec - dailyAET - runoff;
@@ -525,8 +639,10 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
           dailyAET += soil;
           soil = R(0);
         }
-        runoff *= cfa;
-        immediate *= cfa;
+        if (corrected) {
+          runoff *= cfa;
+          immediate *= cfa;
+        }
         const R fgr = c.fg[s] * runoff;
         gwr = cmp::lt(c.rgmax[s], fgr) ? c.rgmax[s] : fgr;
         // the reference's inland-sink test here reads a grid nothing fills (globals.cpp:8),
@@ -534,26 +650,33 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
         if ((flags & F_ARID_GW) && cmp::le(dailyPrec, c.pcritgwa[s])) {
           pot = gwr;
           gwr = R(0);
+          runoff -= pot;
+          soil += pot * c.inv_cfa[s];
         }
-        runoff -= pot;
-        soil += pot * c.inv_cfa[s];
         if (cmp::gt(soil, Smax)) {
           overflow += soil - Smax;
           soil = Smax;
         }
-        overflow *= cfa;
-        total = runoff + immediate + overflow;
+        if (corrected) overflow *= cfa;
+        total = runoff;
+        if (!cmp::is_zero(immediate)) total += immediate;
+        if (!cmp::is_zero(overflow)) total += overflow;
       }
     } else {
-      overflow *= cfa;
-      effPrec *= cfa;
+      if (corrected) {
+        overflow *= cfa;
+        effPrec *= cfa;
+      }
       total += overflow + effPrec;
       dailyAET = R(0);
       leak -= cfa * immediate;   // built-up runoff is dropped in this branch
     }
     gwr_route = gwr;   // G_dailyGwRecharge (daily.cpp:1232)
-    lsc += soil - initialStorage;
-    cellAET = (lsc - dailyPrec) * (cfa - R(1.0)) + (dailyAET + canopyEvapo + snowEvapo) * cfa;
+    cellAET = dailyAET + canopyEvapo + snowEvapo;
+    if (corrected) {
+      lsc += soil - initialStorage;
+      cellAET = (lsc - dailyPrec) * (cfa - R(1.0)) + cellAET * cfa;
+    }
     if (cmp::lt0(cellAET)) {
       neg_land_aet = cellAET;
       cellAET = R(0);
@@ -1133,7 +1256,8 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       rt.e_ow += remRiver0;
       remainingUse = R(0);
     }
-  } else if (cmp::lt0(inflow * omeK + K * S0 * eK)) {   // sign of RivEvapoRemUseMax (routing.cpp:3444-3449)
+  } else if ((cmp::lt0(inflow) || cmp::lt0(S0)) &&
+             cmp::lt0(inflow * omeK + K * S0 * eK)) {   // sign of RivEvapoRemUseMax (routing.cpp:3444-3449)
     const R maxUse = inflow + K * S0 * eK * m::rcp(omeK);   // K >= 1e-5 / length: omeK > 0
     S = R(0);
     transported = inflow + S0 - maxUse;
