@@ -1212,8 +1212,10 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t)16 << 30;
     // (ensembles: 24 GB, so that the ring holds two chunks of the stream overlap)
     const size_t ring_bytes = std::min<size_t>((size_t)(ctx->members > 1 ? 24 : 8) << 30, free_b / 8);
-    // per day: surface runoff and recharge of every state, the three PETs of every cell
-    const size_t budget = opt->ring_days > 0 ? (size_t)opt->ring_days : ring_bytes / (elem * (2 * N + 3 * (size_t)n));
+    // per day: surface runoff and recharge of every state, the PETs of every cell (with
+    // one member two of the three wait in the slots that runoff and recharge overwrite)
+    const bool ens_ring = ctx->members > 1;
+    const size_t budget = opt->ring_days > 0 ? (size_t)opt->ring_days : ring_bytes / (elem * (2 * N + (ens_ring ? 3 : 1) * (size_t)n));
     const int ring = (int)std::max<size_t>(std::max(8, 2 * ctx->days_per_step),
                                            std::min<size_t>(budget, (size_t)ctx->max_days));
     ctx->rd.days_per_step = ctx->rf.days_per_step = ctx->days_per_step;
@@ -1221,8 +1223,8 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
       ctx->rd.ring_days = ring;
       ctx->rd.rs = ctx->alloc<double>((size_t)ring * N);
       ctx->rd.gwr = ctx->alloc<double>((size_t)ring * N);
-      ctx->rd.pet = ctx->alloc<double>((size_t)ring * n);
-      ctx->rd.pet_snow = ctx->alloc<double>((size_t)ring * n);
+      ctx->rd.pet = ctx->rd.rs;   // FP64 contexts have one member
+      ctx->rd.pet_snow = ctx->rd.gwr;
       ctx->rd.pet_water = ctx->alloc<double>((size_t)ring * n);
       if (!ctx->rd.rs || !ctx->rd.gwr || !ctx->rd.pet || !ctx->rd.pet_snow || !ctx->rd.pet_water) return WG_ERR_NOMEM;
       if (opt->water_temp) {   // the river's open-water precipitation of the cells run ahead
@@ -1233,8 +1235,8 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
       ctx->rf.ring_days = ring;
       ctx->rf.rs = ctx->alloc<float>((size_t)ring * N);
       ctx->rf.gwr = ctx->alloc<float>((size_t)ring * N);
-      ctx->rf.pet = ctx->alloc<float>((size_t)ring * n);
-      ctx->rf.pet_snow = ctx->alloc<float>((size_t)ring * n);
+      ctx->rf.pet = ens_ring ? ctx->alloc<float>((size_t)ring * n) : ctx->rf.rs;
+      ctx->rf.pet_snow = ens_ring ? ctx->alloc<float>((size_t)ring * n) : ctx->rf.gwr;
       ctx->rf.pet_water = ctx->alloc<float>((size_t)ring * n);
       if (!ctx->rf.rs || !ctx->rf.gwr || !ctx->rf.pet || !ctx->rf.pet_snow || !ctx->rf.pet_water) return WG_ERR_NOMEM;
     }

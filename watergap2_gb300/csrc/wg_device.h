@@ -221,7 +221,9 @@ struct DevRingT {
   R *rs, *gwr;
   R *owp;                  // open-water precipitation (only with the water temperature, else null)
   // [ring_days][n]: potential evapotranspiration of every cell's land without and
-  // with snow and of open water (k_pet), the same for all members
+  // with snow and of open water (k_pet), the same for all members.  With one member
+  // pet and pet_snow are rs and gwr: the thread that runs a cell-day's vertical
+  // balance reads them and then writes the day's runoff and recharge there
   R *pet, *pet_snow, *pet_water;
   int32_t ring_days;
   int32_t days_per_step;   // days every cell advances per wavefront step (K >= 1)
