@@ -216,6 +216,29 @@ wg_status build_topology(int n, const int32_t *down, const int32_t *rout_order, 
     if (ca != cb) return ca < cb;
     return t.offset[a] < t.offset[b];
   });
+  // A class with water bodies starts a warp of its own, the class before it filled up
+  // with cells of class 0 as far as they go: a warp that straddled two classes ran
+  // both sets of branches, one that straddled the rare combinations of bodies all
+  // of them, and the slowest warp sets the pace of the day (633 cells with every
+  // kind of body, one year: 9.2 -> 7.2 ms).
+  if (cls) {
+    const size_t plain = std::lower_bound(seq.begin(), seq.end(), 1u, [&](int a, uint32_t v) { return cls[a] < v; }) - seq.begin();
+    std::vector<int32_t> packed;
+    packed.reserve(n);
+    size_t used = 0;   // class-0 cells taken as filling, from the end (the largest offsets)
+    for (size_t k = plain; k < (size_t)n;) {
+      size_t e = k;
+      while (e < (size_t)n && cls[seq[e]] == cls[seq[k]]) packed.push_back(seq[e++]);
+      while (packed.size() % 32 && used < plain) packed.push_back(seq[plain - 1 - used++]);
+      k = e;
+    }
+    packed.insert(packed.begin(), seq.begin(), seq.begin() + (plain - used));
+    // whole warps of class 0 stay in front; their remainder goes to the end, so that
+    // the filled warps keep their alignment
+    const size_t front = (plain - used) % 32;
+    std::rotate(packed.begin() + (plain - used - front), packed.begin() + (plain - used), packed.end());
+    seq.swap(packed);
+  }
   const int W = (n + 31) / 32;
   const int wfull = n / 32;   // a partial last warp stays last, so that every full warp stays aligned
   std::vector<uint32_t> wcls(W);
@@ -352,6 +375,10 @@ void join_uploads(wg_ctx *ctx) {
   }
 }
 
+// Days of rows in the outflow buffer of the wavefront that waits for outflows: its
+// launches run up to that many days less one step (the default chunk is 16 days).
+constexpr int kDataDays = 65;
+
 bool valid_block_threads(int threads, int precision, int members) {
   const int mx = members > 1 ? PipeBounds<float, true>::threads
                              : (precision == 0 ? Bounds<double>::threads : Bounds<float>::threads);
@@ -378,14 +405,17 @@ WarpLayout default_layout(wg_ctx *ctx) {
   const int fits_r = ctx->precision == 0 ? pipeline_max_blocks<double>(false, false, wpb * 32)
                                          : pipeline_max_blocks<float>(false, false, wpb * 32);
   if (fits < blocks || fits_r < blocks) return lay;
-  // vertical-balance warps: fill the block to 20 warps (five per sub-partition at
-  // the 96 registers that kernel is built for), if at least two fit, but no more
-  // than it takes for every block to have its share: beyond that the first blocks
-  // to ask take several warps' work, their routing warps fall behind on the FP64
-  // pipe, and every block waits for them at the step barrier (4,096 cells, one
-  // year: 17 warps per block 9.4 ms, 2 warps 5.0 ms)
-  const int room = 20 - wpb, va = std::min(room, (int)((W + blocks - 1) / blocks));
-  if (room >= 2 && pipeline_max_blocks<double>(true, false, (wpb + va) * 32, true) >= blocks) lay.va_warps = va;
+  // vertical-balance warps: fill the block to the 16 warps that kernel is built for
+  // (beside them the idle warp and, once their steps are done, all others run the
+  // vertical balance), but no more than it takes for every block to have its share:
+  // beyond that the first blocks to ask take several warps' work and their routing
+  // warps fall behind on the FP64 pipe (4,096 cells, one year: 17 warps per block
+  // 9.4 ms, 2 warps 5.0 ms)
+  const int room = Bounds<double>::threads / 32 - wpb, va = std::min(room, (int)((W + blocks - 1) / blocks));
+  if (pipeline_max_blocks<double>(true, false, (wpb + va) * 32, true) >= blocks) {
+    lay.va_warps = va;
+    lay.va_on = true;
+  }
   // the idle warp: the last warp of the sub-partition that has the fewest warps
   // (of those that have any: a block of fewer than four warps leaves some empty)
   int cnt[4] = {0, 0, 0, 0};
@@ -952,7 +982,7 @@ static wg_status setup_water_temp(wg_ctx *ctx, const wg_region *r) {
   DevWaterTemp &w = ctx->wt;
   w.temp = ctx->alloc<double>(6 * N);
   w.ice = ctx->alloc<double>(6 * N);
-  w.outt = ctx->alloc<double>((size_t)2 * ctx->days_per_step * N);
+  w.outt = ctx->alloc<double>(ctx->outq_rows() * N);
   w.lw = ctx->alloc<float>((size_t)ctx->max_days * n);
   w.qst_t = ctx->alloc<double>((size_t)ctx->max_days * std::max(1, ctx->nstation));
   if (!w.temp || !w.ice || !w.outt || !w.lw || !w.qst_t) return WG_ERR_NOMEM;
@@ -1106,7 +1136,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
   std::vector<uint32_t> cls(n);
   for (int i = 0; i < n; ++i) cls[i] = work_class(r, i);
   if (!opt->block_threads && ctx->members == 1) ctx->layout = default_layout(ctx.get());
-  ctx->va_warps_default = ctx->layout.va_warps;
+  ctx->va_default = ctx->layout.va_on;
   std::vector<int32_t> node_of;   // GLWD units: a unit's cells are one node of the wavefront
   if (aggr) {
     std::vector<int32_t> order;
@@ -1345,7 +1375,9 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
   // whole state of five snow bands)
   ctx->staging_bytes = std::max<size_t>((size_t)ctx->staging_days * sizeof(float), 30 * sizeof(double)) * n;
   ctx->staging = ctx->alloc<float>(ctx->staging_bytes / sizeof(float));
-  ctx->outq = ctx->alloc<double>((size_t)2 * ctx->days_per_step * N);   // two steps of days
+  // (one member; with GLWD units a cell's upstream cells may be further upstream in steps)
+  ctx->outq_days = ctx->members == 1 && !ctx->glwd.on ? std::max(kDataDays, 2 * ctx->days_per_step) : 0;
+  ctx->outq = ctx->alloc<double>(ctx->outq_rows() * N);
   ctx->qst = ctx->alloc<double>((size_t)ctx->max_days * std::max(1, ctx->nstation) * ctx->members);
   ctx->balance.enabled = opt->record_balance ? 1 : 0;
   ctx->balance.acc = ctx->alloc<double>(ctx->balance.enabled ? (size_t)WG_BALANCE_ARRAYS * N : 1);
@@ -1835,13 +1867,36 @@ wg_status wg_step_routing(wg_ctx *ctx, int32_t doy, int32_t oday) {
 // wavefront launch carries warps that compute the next chunk's, so the FP64 pipe
 // has their work while the routing warps wait on loads and step barriers.  Every
 // call ends with the vertical state exactly at step t_e either way.
+// How the wavefront's steps wait for one another: for the outflows themselves where
+// every cell runs, else at a grid barrier.  A run keeps the buffer that it began with.
+struct StepSync { DevSync sync; double *outq; DevWaterTemp wt; };
+static StepSync step_sync(wg_ctx *ctx, int kd, bool data) {
+  StepSync r{ctx->sync, ctx->outq, ctx->wt};
+  r.sync.rows = 2;
+  r.sync.data = 0;
+  if (data) {
+    const size_t skip = (size_t)2 * ctx->days_per_step * ctx->nstate();
+    r.outq += skip;
+    if (r.wt.outt) r.wt.outt += skip;
+    r.sync.rows = ctx->outq_days / kd;
+    r.sync.data = !ctx->cells_skipped();
+  }
+  return r;
+}
+static bool data_sync_possible(const wg_ctx *ctx) {
+  return ctx->outq_days > 0 && !ctx->sync.flow && !ctx->cells_skipped();
+}
+
 template <class R>
 static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevStateT<R> &s, const DevVertT<R> &v,
                                 DevRingT<R> ring, int kd, int doy0, int fday0, int oday0, int ndays, int t_b,
                                 int t_e) {
   ring.days_per_step = kd;
   const bool ov = ctx->overlap();
-  const int chunk = ctx->eff_chunk(kd);
+  if (t_b == 0) ctx->run_data = data_sync_possible(ctx);
+  const StepSync ss = step_sync(ctx, kd, ctx->run_data);
+  // (waiting for outflows, a launch's steps have rows of their own beside the one before)
+  const int chunk = ss.sync.data ? std::min(ctx->eff_chunk(kd), ss.sync.rows - 1) : ctx->eff_chunk(kd);
   if (ctx->ens_overlap && ctx->members > 1 && ctx->va_stream) {
     // the next chunk's vertical balance on the second stream, beside this chunk's
     // wavefront launch: the vertical balance of chunk k+1 writes ring slots that
@@ -1864,9 +1919,9 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
       const int b = std::min(t_e, a + chunk);
       e = cudaStreamWaitEvent(ctx->stream, ctx->ev_va, 0);
       if (e == cudaSuccess)
-        e = launch_pipeline(true, c, s, v, ctx->forcing, ctx->mem, ctx->balance, ring, ctx->sync, ctx->outq, ctx->qst,
+        e = launch_pipeline(true, c, s, v, ctx->forcing, ctx->mem, ctx->balance, ring, ss.sync, ss.outq, ctx->qst,
                             doy0, fday0, oday0, ndays, a, b, ctx->blocks_fused, ctx->threads, ctx->layout, ctx->mon,
-                            DevVaWork{}, ctx->wt, ctx->wu, ctx->stream);
+                            DevVaWork{}, ss.wt, ctx->wu, ctx->stream);
       ctx->launches++;
       if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_pipe[k & 1], ctx->stream);
       if (e == cudaSuccess && b < t_e) {
@@ -1881,7 +1936,6 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
   }
   DevVaWork vw{};
   vw.next = ctx->va_next;
-  vw.nitems = (int)((ctx->nstate() + 31) / 32);
   int pet_end = t_b;   // the ring holds the PET of the steps before pet_end
   for (int a = t_b; a < t_e; a += chunk) {
     const int b = std::min(t_e, a + chunk);
@@ -1905,10 +1959,11 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
     vw.t_b = b;
     vw.t_e = std::min(t_e, b + chunk);
     vw.warps = (ov && vw.t_e > vw.t_b) ? ctx->layout.va_warps : 0;
+    vw.nitems = (ov && vw.t_e > vw.t_b) ? (int)((ctx->nstate() + 31) / 32) : 0;
     if (e == cudaSuccess)
-      e = launch_pipeline(true, c, s, v, ctx->forcing, ctx->mem, ctx->balance, ring, ctx->sync, ctx->outq, ctx->qst,
+      e = launch_pipeline(true, c, s, v, ctx->forcing, ctx->mem, ctx->balance, ring, ss.sync, ss.outq, ctx->qst,
                           doy0, fday0, oday0, ndays, a, b, ctx->blocks_fused, ctx->threads, ctx->layout, ctx->mon,
-                          vw, ctx->wt, ctx->wu, ctx->stream);
+                          vw, ss.wt, ctx->wu, ctx->stream);
     ctx->launches++;
     if (ev) cudaEventRecord(ev[2], ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "run_steps");
@@ -1946,15 +2001,17 @@ static wg_status routing_now(wg_ctx *ctx, int doy, int oday) {
   cudaSetDevice(ctx->device);
   join_uploads(ctx);
   ctx->launches++;
+  StepSync ss = step_sync(ctx, 1, data_sync_possible(ctx));
+  if (ss.sync.data) ss.sync.rows = 1;   // one day: a cell's outflow is written once
   cudaError_t e = ctx->precision == 0
                       ? launch_pipeline(false, ctx->cd, ctx->sd, ctx->vd, ctx->forcing, ctx->mem, ctx->balance,
-                                        ctx->rd, ctx->sync, ctx->outq, ctx->qst, doy, ctx->last_vertical_fday, oday, 1,
+                                        ctx->rd, ss.sync, ss.outq, ctx->qst, doy, ctx->last_vertical_fday, oday, 1,
                                         0, ctx->topo.nlevel, ctx->blocks_route, ctx->threads, ctx->layout, ctx->mon,
-                                        DevVaWork{}, ctx->wt, ctx->wu, ctx->stream)
+                                        DevVaWork{}, ss.wt, ctx->wu, ctx->stream)
                       : launch_pipeline(false, ctx->cf, ctx->sf, ctx->vf, ctx->forcing, ctx->mem, ctx->balance,
-                                        ctx->rf, ctx->sync, ctx->outq, ctx->qst, doy, ctx->last_vertical_fday, oday, 1,
+                                        ctx->rf, ss.sync, ss.outq, ctx->qst, doy, ctx->last_vertical_fday, oday, 1,
                                         0, ctx->topo.nlevel, ctx->blocks_route, ctx->threads, ctx->layout, ctx->mon,
-                                        DevVaWork{}, ctx->wt, ctx->wu, ctx->stream);
+                                        DevVaWork{}, ss.wt, ctx->wu, ctx->stream);
   return cuda_fail(ctx, e, "step_routing");
 }
 

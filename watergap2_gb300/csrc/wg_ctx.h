@@ -83,6 +83,13 @@ struct wg_ctx {
   bool has_kc = false;                     // the region gave the LCT crop coefficients
   std::vector<double> cell_area, cell_cont;   // cell order: area [km2], continental share [%] as raised
   double *daily_storage_buf = nullptr;     // wg_record_daily_storages (context allocation)
+  // the outflow buffer: two steps of days for the wavefront with a grid barrier, then
+  // outq_days days of rows for the one that waits for the outflows themselves
+  // (DevSync::data; 0: none), the water temperature's outt likewise
+  int outq_days = 0;
+  bool run_data = false;                   // which of the two the run in progress uses
+  size_t outq_rows() const { return (size_t)2 * days_per_step + outq_days; }
+  bool cells_skipped() const { return (precision == 0 ? cd.active : cf.active) != nullptr; }
   double *outq = nullptr, *qst = nullptr, *vol0 = nullptr, *partial = nullptr;
   float *staging = nullptr;
   float *staging_async = nullptr;          // staging of wg_upload_forcing_async
@@ -121,7 +128,7 @@ struct wg_ctx {
     bool vpending = false;                 // a vertical call waiting for its routing call
     int vdoy = 0, vfday = 0;
   } defer;
-  int va_warps_default = 0;                // vertical-balance warps the layout was sized for
+  bool va_default = false;                 // the layout has room for the vertical balance
   unsigned int *va_next = nullptr;         // their work counter
   Snapshot *snap = nullptr;                // device copy of the mutable state (autotuner)
   cudaGraph_t graph = nullptr;             // wg_graph_capture
@@ -180,7 +187,7 @@ struct wg_ctx {
   // longest chunk of wavefront steps (of kd days) one launch pair may run: its days fit the ring
   int max_chunk(int kd) const { return ring_days() / kd; }
   // the wavefront launches carry vertical-balance warps for the next chunk
-  bool overlap() const { return layout.va_warps > 0 && layout.idle_warp >= 0 && threads == layout.threads; }
+  bool overlap() const { return layout.va_on && layout.idle_warp >= 0 && threads == layout.threads; }
   // longest chunk: with the overlap the ring holds this chunk's and the next one's days
   int chunk_cap(int kd) const { return (overlap() || ens_overlap) ? max_chunk(kd) / 2 : max_chunk(kd); }
   int chunk_cap() const { return chunk_cap(days_per_step); }

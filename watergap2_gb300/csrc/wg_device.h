@@ -235,7 +235,7 @@ struct DevRingT {
 struct DevWaterTemp {
   double *temp;              // [6][N] the previous day's temperatures [degC]
   double *ice;               // [6][N] ice thickness [km] (-9999 where a water body has none)
-  double *outt;              // [2][days_per_step][N] river temperature of the step, read downstream
+  double *outt;              // [rows][days_per_step][N] river temperature of the step, read downstream
   const float *lw;           // [max_days][n] downward longwave radiation [W/m2]
   const float *gwt;          // [n] yearly groundwater temperature [degC]
   const double *len_check;   // [n] river length as read (55: no river in the cell)
@@ -282,6 +282,11 @@ struct DevVaWork {
   int32_t warps, t_b, t_e, nitems;
 };
 
+// An outflow buffer's entry that no step has written: a NaN with all bits set, which
+// no arithmetic gives (results are canonical NaNs; a stored value with these bits
+// would be made one).
+constexpr unsigned long long kNoOutflow = ~0ull;
+
 struct DevSync {
   unsigned int *counter;   // monotonic arrival counter of the grid barrier
   int *error;              // 0 ok, nonzero: a barrier wait exceeded its limit (WG_ERR_TIMEOUT)
@@ -292,8 +297,14 @@ struct DevSync {
   int *wstep;
   const int32_t *dep_ptr, *dep_idx;
   int32_t nwarps, flow;
+  // outflow as its own signal (data != 0): the rows of the outflow buffer that the
+  // launch's steps write hold kNoOutflow before it, a cell that needs an upstream
+  // cell's outflow of the step before waits until the value is there, and there is
+  // no barrier between steps.  rows: the buffer's rows, step t in row t % rows
+  int32_t rows, data;
   // failure-detection test: arrivals the grid barrier waits for beyond the grid's
-  // blocks (0 in every run; 1 makes each wait run out, see wg_set_barrier_test)
+  // blocks, and with data nonzero values not taken for outflow (0 in every run; 1
+  // makes each wait run out, see wg_set_barrier_test)
   uint32_t extra_arrivals;
 };
 

@@ -87,6 +87,57 @@ __device__ __forceinline__ bool grid_barrier(const DevSync &sync, unsigned round
   return s_ok != 0;
 }
 
+// An outflow (or river temperature) of the step before, which another thread writes.
+// With sync.data it is its own signal: one 64-bit word, written and read with
+// relaxed gpu-scope accesses, so that no ordering between words matters and no
+// acquire empties the SM's L1 cache (the grid barrier's did, and every constant and
+// state of the next step came back from L2).  The wait is bounded like the grid
+// barrier's: when it runs out the error word is set and the caller stops.
+#define WG_DATA_SPIN_LIMIT (1u << 20)
+#ifndef WG_POLL_NS
+#define WG_POLL_NS 100
+#endif
+
+__device__ __forceinline__ double ld_relaxed(const double *p) {
+  double v;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void st_outflow(double *p, double v) {
+  if ((unsigned long long)__double_as_longlong(v) == kNoOutflow) v = __longlong_as_double(0x7ff8000000000000ll);
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+
+__device__ __forceinline__ bool is_outflow(const DevSync &sync, double v) {
+  return (unsigned long long)__double_as_longlong(v) != kNoOutflow && !sync.extra_arrivals;
+}
+__device__ __forceinline__ bool has_outflow(const DevSync &sync, const double *p) { return is_outflow(sync, ld_relaxed(p)); }
+
+// One more poll of a warp (converged) or thread: true when the wait has run out, here
+// or elsewhere in the grid.
+__device__ __forceinline__ bool wait_ran_out(const DevSync &sync, unsigned &it) {
+  if (++it <= WG_DATA_SPIN_LIMIT && ((it & 255u) != 0u || !*(volatile int *)sync.error)) return false;
+  atomicExch(sync.error, 1);
+  return true;
+}
+
+// The outflow itself.  WAIT (the per-day routing call, whose lanes each route one
+// cell once): waiting for it if need be, failed when the wait runs out.  Else it is
+// there, or belongs to an upstream cell that does not run.
+template <bool WAIT>
+__device__ __forceinline__ double upstream_value(const DevSync &sync, const double *p, bool &failed) {
+  double v = ld_relaxed(p);
+  if constexpr (WAIT) {
+    unsigned it = 0;
+    while (sync.data && !failed && ((unsigned long long)__double_as_longlong(v) == kNoOutflow || sync.extra_arrivals)) {
+      failed = wait_ran_out(sync, it);
+      v = ld_relaxed(p);
+    }
+  }
+  return (unsigned long long)__double_as_longlong(v) == kNoOutflow ? 0. : v;
+}
+
 __device__ __forceinline__ int ld_acquire_int(const int *p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -207,6 +258,12 @@ __device__ __forceinline__ Radiation<R> radiation_at(const DevCellsT<R> &c, int 
   return radiation<R>(c, s, Tf, SWf, c.ext_rad[ti], c.inv_s0[ti]);
 }
 
+// Row of the ring for day d (a division only where the run is longer than the ring).
+template <class R>
+__device__ __forceinline__ size_t ring_row(const DevRingT<R> &ring, int d) {
+  return (size_t)(d < ring.ring_days ? d : d % ring.ring_days);
+}
+
 template <class R>
 __device__ __forceinline__ Pet<R> ring_pet(const DevRingT<R> &ring, size_t k) {
   return Pet<R>{ring.pet[k], ring.pet_snow[k], ring.pet_water[k]};
@@ -233,7 +290,7 @@ __global__ void __launch_bounds__(256) k_pet(DevCellsT<R> c, DevForcing f, DevRi
   const int d0 = (int)max(0ll, first);
   const int d1 = (int)min(min(first + kPetDays, (long long)kd * (t_e - c.offset[s])), (long long)ndays);
   for (int d = d0; d < d1; ++d) {
-    const size_t fo = (size_t)(fday0 + d) * c.n + s, k = (size_t)(d % ring.ring_days) * c.n + s;
+    const size_t fo = (size_t)(fday0 + d) * c.n + s, k = ring_row(ring, d) * c.n + s;
     const Pet<R> p = pet_of<R>(c, s, radiation_at<R>(c, s, (doy0 - 1 + d) % 365 + 1, f.temp[fo], f.swrad[fo]));
     ring.pet[k] = p.land;
     ring.pet_snow[k] = p.snow;
@@ -314,7 +371,7 @@ __device__ __forceinline__ void va_cell(const DevCellsT<R> &c, const DevStateT<R
     const int doy = (doy0 - 1 + d) % 365 + 1;
     const size_t fo = (size_t)(fday0 + d) * n + s;
     const float Tf = f.temp[fo];
-    const Pet<R> pet = ring_pet(ring, (size_t)(d % ring.ring_days) * n + s);
+    const Pet<R> pet = ring_pet(ring, ring_row(ring, d) * n + s);
     VOut<R> o;
     VSink vs;
     if (!ENS && mon && vert_sink(*mon, oday0 + d, i, N, vs)) {   // the output grids (FP64 single member)
@@ -326,7 +383,7 @@ __device__ __forceinline__ void va_cell(const DevCellsT<R> &c, const DevStateT<R
       vertical_cell<R>(c, s, gam, canopy, soil, gsnow, st.snow_band + i, N, days, status, psum, laf, laf,
                        R(f.prec[fo]) * pf, Tf, pet, o);
     }
-    const size_t ri = (size_t)(d % ring.ring_days) * N + i;
+    const size_t ri = ring_row(ring, d) * N + i;
     ring.rs[ri] = o.rs;
     ring.gwr[ri] = o.gwr;
     if (ring.owp) ring.owp[ri] = o.owp;   // the river's, for the water temperature
@@ -380,22 +437,8 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
   const int n = c.n;
   const int M = ENS ? mem.members : 1;
   const size_t N = (size_t)n * M;
-  if (VAW && (int)(threadIdx.x >> 5) >= (int)(blockDim.x >> 5) - vw.warps) {
-    // the block's last vw.warps warps: vertical balance ahead for the next launch's
-    // steps, 32 slots at a time from a shared counter, filling the FP64 pipe while
-    // the routing warps wait on loads and step barriers
-    const unsigned lane = threadIdx.x & 31;
-    for (;;) {
-      unsigned g = 0;
-      if (lane == 0) g = atomicAdd(vw.next, 1u);
-      g = __shfl_sync(0xffffffffu, g, 0);
-      if (g >= (unsigned)vw.nitems) break;
-      const size_t i = (size_t)g * 32 + lane;
-      if (i < N) va_cell<R, ENS>(c, st, f, mem, b, ring, doy0, fday0, ndays, vw.t_b, vw.t_e, i, N, VO ? &mon : nullptr,
-                                 oday0);
-    }
-    return;
-  }
+  // the block's last vw.warps warps run no routing
+  const bool va_only = VAW && (int)(threadIdx.x >> 5) >= (int)(blockDim.x >> 5) - vw.warps;
   const int route_threads = VAW ? (int)blockDim.x - 32 * vw.warps : (int)blockDim.x;
 
   const int kd = FUSED ? ring.days_per_step : 1;   // days per step (the per-day routing call: one)
@@ -419,22 +462,96 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
   // registers for the whole launch instead took ~32 registers per thread, which
   // the wavefront launch with vertical-balance warps (96 registers per thread)
   // paid in spills, and measured ~1 % slower on the global grid.
-  for (int t = t_b; t < t_e; ++t) {
+  // waiting for outflows, one cell per thread and one day per step (the shape of every
+  // single-member FP64 run): what the wait reads of the topology stays in registers,
+  // the day's ring values are loaded before the wait and the outflows it has seen are
+  // the day's inflow, so that one trip to L2 lies between two steps instead of three
+  const bool one = FUSED && !ENS && !GL && sync.data && kd == 1 && gstride >= (long long)N;
+  int one_off = 0, one_u = 0, one_ue = 0, one_up = 0;
+  if (one && gtid < (long long)N) {
+    one_off = c.offset[gtid];
+    one_u = c.up_ptr[gtid];
+    one_ue = c.up_ptr[gtid + 1];
+    if (one_ue > one_u) one_up = c.up_idx[one_u];
+  }
+  int row_t = t_b % sync.rows;   // t % sync.rows
+  for (int t = va_only ? t_e : t_b; t < t_e; ++t, row_t = row_t + 1 == sync.rows ? 0 : row_t + 1) {
     if (flow && t > t_b) {
       if (!wait_deps(sync, wpos, t - t_b - 1)) return;
       __syncwarp();   // the lanes that acquired the flags order the others' loads
     }
     if (kd * (t - c.nlevel + 1) < ndays) {   // some cell still has a day to compute
-      double *q_now0 = outq + (size_t)(t & 1) * kd * N;
-      const double *q_prev0 = outq + (size_t)((t + 1) & 1) * kd * N;
-      double *t_now0 = WT ? wtp.outt + (size_t)(t & 1) * kd * N : nullptr;   // river temperature, same slots
-      const double *t_prev0 = WT ? wtp.outt + (size_t)((t + 1) & 1) * kd * N : nullptr;
+      const size_t row = (size_t)row_t * kd * N, prev_row = (size_t)(row_t ? row_t - 1 : sync.rows - 1) * kd * N;
+      double *q_now0 = outq + row;
+      const double *q_prev0 = outq + prev_row;
+      double *t_now0 = WT ? wtp.outt + row : nullptr;   // river temperature, same slots
+      const double *t_prev0 = WT ? wtp.outt + prev_row : nullptr;
+      [[maybe_unused]] R pre_rs = R(0), pre_gwr = R(0);
+      [[maybe_unused]] double pre_up = 0., pre_e = 0.;
+      if (one) {
+        int k = 0, k_e = 0;
+        const int d = t - one_off;
+        if (gtid < (long long)N && d >= 0 && d < ndays) {
+          const size_t ri = ring_row(ring, d) * N + (size_t)gtid;
+          pre_rs = ring.rs[ri];
+          pre_gwr = ring.gwr[ri];
+          k = one_u;
+          k_e = one_ue;
+        }
+        unsigned it = 0;
+        for (;;) {
+          while (k < k_e) {
+            const size_t ui = k == one_u ? one_up : c.up_idx[k];
+            const double q = ld_relaxed(q_prev0 + ui);
+            double tq = 0.;
+            if constexpr (WT) tq = ld_relaxed(t_prev0 + ui);
+            if (!is_outflow(sync, q) || (WT && !is_outflow(sync, tq))) break;
+            pre_up += q;
+            if constexpr (WT) pre_e += q * WT_RC * (tq + WT_CONV_K);
+            ++k;
+          }
+          if (__all_sync(0xffffffffu, k >= k_e)) break;
+          if (wait_ran_out(sync, it)) return;
+          __nanosleep(WG_POLL_NS);
+        }
+      } else if (FUSED && !ENS && !GL && sync.data) {
+        // the whole warp waits here, converged, for the outflows its cells need: a
+        // wait lane by lane inside the cell's routing split the warps, and each part
+        // then ran the rest of the step by itself (global grid, one year: 32 ms)
+        for (long long i = gtid; __any_sync(0xffffffffu, i < (long long)N); i += gstride) {
+          int u = 0, u_e = 0, left = 0;
+          const double *p = q_prev0, *pt = t_prev0;
+          if (i < (long long)N) {
+            const int dbase = kd * (t - c.offset[i]);
+            if (dbase >= 0 && dbase < ndays) {
+              u = c.up_ptr[i];
+              u_e = c.up_ptr[i + 1];
+              left = u_e > u ? min(kd, ndays - dbase) : 0;
+            }
+          }
+          unsigned it = 0;
+          int k = u;
+          for (;;) {   // day by day of the step, upstream cell by upstream cell
+            while (left > 0 && has_outflow(sync, p + c.up_idx[k]) && (!WT || has_outflow(sync, pt + c.up_idx[k]))) {
+              if (++k == u_e) {
+                k = u;
+                p += N;
+                if constexpr (WT) pt += N;
+                --left;
+              }
+            }
+            if (__all_sync(0xffffffffu, left == 0)) break;
+            if (wait_ran_out(sync, it)) return;
+            __nanosleep(WG_POLL_NS);
+          }
+        }
+      }
       // state index i always belongs to thread i mod gstride, so a cell's state is read
       // and written by one thread; only upstream outflows cross threads (read via L2)
       for (long long i = gtid; i < (long long)N; i += gstride) {
         const int s0 = ENS ? (int)(i / M) : (int)i;
         const int mm = ENS ? (int)(i - (long long)s0 * M) : 0;
-        const int dbase = kd * (t - c.offset[s0]);
+        const int dbase = kd * (t - (one ? one_off : c.offset[s0]));
         if (dbase < 0 || dbase >= ndays) continue;   // this cell's wavefront has not reached it yet / is done
         // a GLWD unit whose riparian cells' use its outflow cell meets (GL) is routed
         // by the thread of its first cell in routing order, cell by cell in that
@@ -469,9 +586,9 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
           const R laf = st.laf[si];
           const R laf_prev = st.laf_prev[si];
           if (FUSED && !(fl & F_VINLINE)) {
-            const size_t ri = (size_t)(d % ring.ring_days) * N + si;
-            o.rs = ring.rs[ri];
-            o.gwr = ring.gwr[ri];
+            const size_t ri = ring_row(ring, d) * N + si;
+            o.rs = one ? pre_rs : ring.rs[ri];
+            o.gwr = one ? pre_gwr : ring.gwr[ri];
             o.transfer = R(0); o.owp = R(0); o.owpet = R(0);
             o.land_in = R(0); o.land_evap = R(0); o.land_leak = R(0);   // accounted ahead
             if constexpr (WT) {
@@ -498,7 +615,9 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
               vk[3 * N] = vk[4 * N] + fll * 100. + vk[5 * N];
             }
             const float Tf = f.temp[fo];
-            const Pet<R> pet = ring_pet(ring, (size_t)(d % ring.ring_days) * n + s);
+            // (with one member the ring's runoff and recharge slots hold the land's PETs)
+            const size_t rk = ring_row(ring, d) * n + s;
+            const Pet<R> pet = one ? Pet<R>{pre_rs, pre_gwr, ring.pet_water[rk]} : ring_pet(ring, rk);
             const R prev = started == 1 ? laf_prev : laf;   // daily.cpp:159-169
             if (VO && vo) {
               const Radiation<R> rad = radiation_at<R>(c, s, doy, Tf, f.swrad[fo]);
@@ -511,17 +630,28 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
             o.rs = v.rs[s]; o.gwr = v.gwr[s]; o.transfer = v.transfer[s]; o.owp = v.owp[s]; o.owpet = v.owpet[s];
             o.land_in = v.land_in[s]; o.land_evap = v.land_evap[s]; o.land_leak = v.land_leak[s];
           }
-          // upstream inflow, summed in FP64 in the reference's push order (routing.cpp:3955-3958)
+          // upstream inflow, summed in FP64 in the reference's push order
+          // (routing.cpp:3955-3958), when routing asks for it
           double up = 0., e_up = 0.;
-          const int u0 = c.up_ptr[s], u1 = c.up_ptr[s + 1];
-          for (int k = u0; k < u1; ++k) {
-            const size_t ui = (size_t)c.up_idx[k] * M + mm;
-            // an upstream cell of the same unit was routed this step, earlier in this loop
-            const double qu = (GL && unit >= 0 && wu.unit_of[c.up_idx[k]] == unit) ? q_now[ui] : __ldcg(q_prev + ui);
-            up += qu;
-            if constexpr (WT)   // the energy the inflow carries (calcWaterTemp.cpp:76-83)
-              e_up += qu * WT_RC * (__ldcg(t_prev0 + (size_t)kk * N + ui) + WT_CONV_K);
+          bool failed = false;
+          const int u0 = one ? 0 : c.up_ptr[s], u1 = one ? 0 : c.up_ptr[s + 1];
+          if (one) {
+            up = pre_up;
+            e_up = pre_e;
           }
+          auto inflow_up = [&]() -> double {
+            for (int k = u0; k < u1; ++k) {
+              const size_t ui = (size_t)c.up_idx[k] * M + mm;
+              // an upstream cell of the same unit was routed this step, earlier in this loop
+              const double qu = (GL && unit >= 0 && wu.unit_of[c.up_idx[k]] == unit)
+                                    ? q_now[ui] : upstream_value<!FUSED>(sync, q_prev + ui, failed);
+              up += qu;
+              if constexpr (WT)   // the energy the inflow carries (calcWaterTemp.cpp:76-83)
+                e_up += qu * WT_RC * (upstream_value<!FUSED>(sync, t_prev0 + (size_t)kk * N + ui, failed) + WT_CONV_K);
+            }
+            return up;
+          };
+          if constexpr (WT) inflow_up();   // the water temperature's day begins with it
           RState<R> rs = load_rstate(st, si, fl);
           RTerms<R> rt;
           // the water temperature (routing.cpp:4241-4513) body by body inside
@@ -550,19 +680,21 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
             // storages stay, nothing flows on, and the inflow stays behind in
             // G_riverInflow, i.e. leaves the system (a negative leak: the leak
             // counts water the model adds)
+            if constexpr (!WT) inflow_up();
             tv = R(0);
             rt.p_ow = R(0); rt.e_ow = R(0); rt.leak = R(-up); rt.velocity = R(0);
           } else {
-            tv = routing_cell<R, WT, WU, GL, RO>(c, s, rs, doy, month, laf, laf_prev, o, up, rt, &wtd, &wu, wrow, si,
-                                                 N, &ro);
+            tv = routing_cell<R, WT, WU, GL, RO>(c, s, rs, doy, month, laf, laf_prev, o,
+                                                 [&]() { return WT ? up : inflow_up(); }, rt, &wtd, &wu, wrow, si, N, &ro);
+            if (!FUSED && failed) return;
             store_rstate(st, si, rs, fl);
           }
-          q_now[si] = (double)tv;
+          st_outflow(q_now + si, (double)tv);
           if constexpr (WT) {
             // a cell without continental area keeps the reference's initial 15 degrees (routing.cpp:174)
             const double tr = nocont ? 15. : wtd.river((double)rs.river, (double)c.bw[s], (double)c.rlen[s],
                                                        (double)c.cfa[s], (double)o.owpet);
-            t_now0[(size_t)kk * N + si] = tr;
+            st_outflow(t_now0 + (size_t)kk * N + si, tr);
             const int stw = c.station[s];
             if (stw >= 0) wtp.qst_t[(size_t)(oday0 + d) * c.nstation + stw] = tr;
           }
@@ -695,8 +827,25 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
       __threadfence();
       __syncwarp();
       if ((threadIdx.x & 31) == 0) st_release_int(sync.wstep + wpos, t - t_b);
-    } else if (t + 1 < t_e) {
+    } else if (!sync.data && t + 1 < t_e) {
       if (!grid_barrier(sync, (unsigned)(t - t_b), route_threads)) return;
+    }
+  }
+  if constexpr (VAW) {
+    // vertical balance ahead for the next launch's steps, 32 slots at a time from a
+    // shared counter: by the block's vw.warps warps from the start, filling the FP64
+    // pipe while the routing warps wait, and by the routing warps once their steps
+    // are done (global grid, one year: five warps that do nothing else 17.5 ms, one
+    // such warp, the idle warp and this help 17.2 ms)
+    const unsigned lane = threadIdx.x & 31;
+    for (;;) {
+      unsigned g = 0;
+      if (lane == 0) g = atomicAdd(vw.next, 1u);
+      g = __shfl_sync(0xffffffffu, g, 0);
+      if (g >= (unsigned)vw.nitems) break;
+      const size_t i = (size_t)g * 32 + lane;
+      if (i < N) va_cell<R, ENS>(c, st, f, mem, b, ring, doy0, fday0, ndays, vw.t_b, vw.t_e, i, N, VO ? &mon : nullptr,
+                                 oday0);
     }
   }
 }
@@ -992,10 +1141,21 @@ cudaError_t launch_pipeline(bool fused, const DevCellsT<R> &c, const DevStateT<R
                             const DevSync &sync, double *outq, double *qst, int doy0, int fday0, int oday0, int ndays,
                             int t_b, int t_e, int blocks, int threads, const WarpLayout &lay, const DevMonthly &mon,
                             const DevVaWork &vw, const DevWaterTemp &wtp, const DevWaterUse &wu, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(sync.counter, 0, sizeof(unsigned), st);
+  cudaError_t e = cudaSuccess;
+  if (sync.data) {   // the rows of this launch's steps: no outflow yet
+    const size_t row = (size_t)(fused ? ring.days_per_step : 1) * c.n * sizeof(double);
+    const int steps = std::min(t_e - t_b, sync.rows), first = t_b % sync.rows, head = std::min(steps, sync.rows - first);
+    for (char *p : {(char *)outq, (char *)(wtp.enabled ? wtp.outt : nullptr)}) {
+      if (!p) continue;
+      if (e == cudaSuccess) e = cudaMemsetAsync(p + first * row, 0xff, head * row, st);
+      if (e == cudaSuccess && steps > head) e = cudaMemsetAsync(p, 0xff, (steps - head) * row, st);
+    }
+  } else {
+    e = cudaMemsetAsync(sync.counter, 0, sizeof(unsigned), st);
+  }
   if (e == cudaSuccess && sync.flow && sync.wstep)
     e = cudaMemsetAsync(sync.wstep, 0xff, (size_t)sync.nwarps * sizeof(int), st);   // -1: no step done yet
-  const bool vaw = fused && vw.warps > 0;
+  const bool vaw = fused && vw.nitems > 0;
   if (e == cudaSuccess && vaw) e = cudaMemsetAsync(vw.next, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
   int cell_warps = lay.cell_warps, idle_warp = mem.members > 1 ? -1 : lay.idle_warp;
@@ -1004,7 +1164,7 @@ cudaError_t launch_pipeline(bool fused, const DevCellsT<R> &c, const DevStateT<R
   // vertical-balance warps only on the single-member layout they were sized for
   if (vaw && (idle_warp < 0 || mem.members > 1 || vw.warps != lay.va_warps)) return cudaErrorInvalidConfiguration;
   DevVaWork vwk = vw;
-  if (!vaw) vwk.warps = 0;
+  if (!vaw) vwk.warps = vwk.nitems = 0;
   void *args[] = {(void *)&c,    (void *)&s,    (void *)&v,     (void *)&f,     (void *)&mem,   (void *)&b,
                   (void *)&ring, (void *)&sync, (void *)&outq,  (void *)&qst,   (void *)&doy0,  (void *)&fday0,
                   (void *)&oday0, (void *)&ndays, (void *)&t_b, (void *)&t_e, (void *)&cell_warps,

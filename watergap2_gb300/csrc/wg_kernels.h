@@ -23,10 +23,10 @@ template <> struct VaBounds<float, true> { static constexpr int threads = 256, m
 // per block and 64 registers, so that an SM holds 32 warps of it (no spills)
 template <class R, bool ENS> struct PipeBounds : Bounds<R> {};
 template <> struct PipeBounds<float, true> { static constexpr int threads = 128, min_blocks = 8; };
-// the single-member FP64 wavefront with vertical-balance warps in the same block:
-// up to 20 warps (5 per SM sub-partition, 96 registers each)
+// the single-member FP64 wavefront with vertical-balance warps in the same block: 16
+// warps, four per SM sub-partition, so that a thread has 128 registers
 template <class R, bool ENS, bool VAW> struct WaveBounds : PipeBounds<R, ENS> {};
-template <class R> struct WaveBounds<R, false, true> { static constexpr int threads = 640, min_blocks = 1; };
+template <class R> struct WaveBounds<R, false, true> { static constexpr int threads = 512, min_blocks = 1; };
 
 // Thread-to-slot layout of the single-member wavefront: each block runs
 // cell_warps warps of 32 consecutive slots plus one idle warp at warp index
@@ -34,7 +34,8 @@ template <class R> struct WaveBounds<R, false, true> { static constexpr int thre
 struct WarpLayout {
   int cell_warps = 0;
   int idle_warp = -1;
-  int va_warps = 0;    // vertical-balance warps appended to each wavefront block (0: none)
+  int va_warps = 0;    // vertical-balance warps appended to each wavefront block
+  bool va_on = false;  // the wavefront launches carry the next chunk's vertical balance
   int blocks = 0;
   int threads = 0;
 };

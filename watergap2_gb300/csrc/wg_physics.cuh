@@ -853,8 +853,9 @@ __device__ __forceinline__ void wu_year_end(double *w, size_t N) {
 }
 
 // One cell of routingClass::routing (routing.cpp:1835-4520) given the vertical
-// outputs and the summed upstream inflow (FP64 for every precision); returns the
-// transported volume.  WT (FP64): the water temperature of each water body runs
+// outputs and the summed upstream inflow (FP64 for every precision; asked for once
+// the cell's groundwater, local lake and local wetland are done, since the caller
+// may have to wait for it); returns the transported volume.  WT (FP64): the water temperature of each water body runs
 // through wtd as soon as the body's routing is done (the reference reads the
 // same terms after the cell's routing, routing.cpp:4287-4356: each body's
 // storage before the day, its evaporation after any reduction, its reduction
@@ -862,9 +863,9 @@ __device__ __forceinline__ void wu_year_end(double *w, size_t N) {
 // wu points at the tables (per cell: slot s, stride c.n) and the state (per
 // member: state index si, stride NN), wrow is the offset of the day's table row.
 // RO: the terms of routing's output grids into *ro.
-template <class R, bool WT = false, bool WU = false, bool GL = false, bool RO = false>
+template <class R, bool WT = false, bool WU = false, bool GL = false, bool RO = false, class UP>
 __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R> &st, int doy, int month, R laf,
-                                          R laf_prev, const VOut<R> &v, double inflow_up, RTerms<R> &rt,
+                                          R laf_prev, const VOut<R> &v, UP &&inflow_up, RTerms<R> &rt,
                                           wt::WtDay *wtd = nullptr, const DevWaterUse *wu = nullptr, size_t wrow = 0,
                                           size_t si = 0, size_t NN = 0, RoutOut *ro = nullptr) {
   typedef M<R> m;
@@ -1017,7 +1018,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     st.locwetl = S;
     st.rf_locwetl = r < R(0) ? R(0) : (r > R(1) ? R(1) : r);
   }
-  inflow = R((double)inflow + inflow_up);   // routing.cpp:2623-2624
+  inflow = R((double)inflow + inflow_up());   // routing.cpp:2623-2624
   if constexpr (WT) wtd->locals_done();
   if (fl & F_GLOLAKE) {  // global lake (routing.cpp:2630-2804)
     const R S0 = st.glolake, maxS = c.maxs_gl[s], rf = st.rf_glolake;

@@ -25,6 +25,7 @@ struct Snapshot {
   std::vector<std::pair<void *, size_t>> fields;   // (device array, bytes)
   char *buf = nullptr;
   size_t bytes = 0;
+  bool run_data = false;                           // wg_ctx::run_data
 };
 
 namespace {
@@ -45,13 +46,13 @@ void list_fields(wg_ctx *ctx, const DevStateT<R> &s, Snapshot &sn) {
   WG_STATE_I(X)
 #undef X
   sn.fields.push_back({(void *)s.snow_band, N * ctx->nband * sizeof(R)});
-  sn.fields.push_back({(void *)ctx->outq, 2 * (size_t)ctx->days_per_step * N * sizeof(double)});
+  sn.fields.push_back({(void *)ctx->outq, ctx->outq_rows() * N * sizeof(double)});
   if (ctx->balance.enabled) sn.fields.push_back({(void *)ctx->balance.acc, WG_BALANCE_ARRAYS * N * sizeof(double)});
   if (ctx->wu.enabled) sn.fields.push_back({(void *)ctx->wu.st, (size_t)wg::WU_NSTATE * N * sizeof(double)});
   if (ctx->wt.enabled) {
     sn.fields.push_back({(void *)ctx->wt.temp, 6 * N * sizeof(double)});
     sn.fields.push_back({(void *)ctx->wt.ice, 6 * N * sizeof(double)});
-    sn.fields.push_back({(void *)ctx->wt.outt, 2 * (size_t)ctx->days_per_step * N * sizeof(double)});
+    sn.fields.push_back({(void *)ctx->wt.outt, ctx->outq_rows() * N * sizeof(double)});
   }
 }
 
@@ -68,6 +69,7 @@ wg_status snapshot_save(wg_ctx *ctx) {
     }
     ctx->snap = sn;
   }
+  ctx->snap->run_data = ctx->run_data;
   size_t off = 0;
   for (auto &f : ctx->snap->fields) {
     cudaError_t e = cudaMemcpyAsync(ctx->snap->buf + off, f.first, f.second, cudaMemcpyDeviceToDevice, ctx->stream);
@@ -79,6 +81,7 @@ wg_status snapshot_save(wg_ctx *ctx) {
 
 wg_status snapshot_restore(wg_ctx *ctx) {
   if (!ctx->snap) return WG_ERR_INVALID;
+  ctx->run_data = ctx->snap->run_data;
   size_t off = 0;
   for (auto &f : ctx->snap->fields) {
     cudaError_t e = cudaMemcpyAsync(f.first, ctx->snap->buf + off, f.second, cudaMemcpyDeviceToDevice, ctx->stream);
@@ -168,18 +171,18 @@ wg_status wg_set_vertical_overlap(wg_ctx *ctx, int32_t enable) {
     return WG_OK;
   }
   if (!enable) {
-    ctx->layout.va_warps = 0;
+    ctx->layout.va_on = false;
     return WG_OK;
   }
-  if (ctx->va_warps_default <= 0 || ctx->layout.idle_warp < 0 || ctx->threads != ctx->layout.threads)
+  if (!ctx->va_default || ctx->layout.idle_warp < 0 || ctx->threads != ctx->layout.threads)
     return WG_ERR_UNSUPPORTED;
-  ctx->layout.va_warps = ctx->va_warps_default;
+  ctx->layout.va_on = true;
   return WG_OK;
 }
 
 int32_t wg_get_vertical_overlap(const wg_ctx *ctx) {
   if (ctx && ctx->members > 1) return ctx->ens_overlap ? 1 : 0;
-  return ctx && ctx->overlap() ? ctx->layout.va_warps : 0;
+  return ctx && ctx->overlap() ? std::max(1, ctx->layout.va_warps) : 0;   // (the idle warp)
 }
 
 int32_t wg_get_chunk_steps(const wg_ctx *ctx) {
@@ -234,12 +237,12 @@ wg_status wg_autotune(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t ndays, i
   // first the context's own shape and layout; with vertical-balance warps, also
   // the same layout without them
   ths.insert(ths.begin(), -1);
-  if (lay0.va_warps > 0) ths.insert(ths.begin() + 1, -2);
-  int best_va = lay0.va_warps;
+  if (lay0.va_on) ths.insert(ths.begin() + 1, -2);
+  bool best_va = lay0.va_on;
   for (int th : ths) {
     if (th < 0) {
       restore_shape0();
-      if (th == -2) ctx->layout.va_warps = 0;
+      if (th == -2) ctx->layout.va_on = false;
     } else if (wg_launch_shape(ctx, th, 0) != WG_OK) {
       continue;   // does not fit the device
     }
@@ -268,7 +271,7 @@ wg_status wg_autotune(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t ndays, i
           best = ms;
           best_th = th;
           best_ch = ch;
-          best_va = ctx->layout.va_warps;
+          best_va = ctx->layout.va_on;
           best_eo = ov.on;
           best_blocks = ctx->blocks_fused;
         }
@@ -292,7 +295,7 @@ wg_status wg_autotune(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t ndays, i
   }
   if (best_th < 0) {
     restore_shape0();
-    ctx->layout.va_warps = best_va;
+    ctx->layout.va_on = best_va;
   } else {
     wg_launch_shape(ctx, best_th, 0);
   }
