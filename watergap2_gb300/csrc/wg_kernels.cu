@@ -376,11 +376,11 @@ __device__ __forceinline__ void va_cell(const DevCellsT<R> &c, const DevStateT<R
     VSink vs;
     if (!ENS && mon && vert_sink(*mon, oday0 + d, i, N, vs)) {   // the output grids (FP64 single member)
       const Radiation<R> rad = radiation_at<R>(c, s, doy, Tf, f.swrad[fo]);
-      vertical_cell<R, std::is_same<R, double>::value>(c, s, gam, canopy, soil, gsnow, st.snow_band + i, N, days,
+      vertical_cell<R, std::is_same<R, double>::value, true>(c, s, gam, canopy, soil, gsnow, st.snow_band + i, N, days,
                                                         status, psum, laf, laf, R(f.prec[fo]) * pf, Tf, pet, o, &vs,
                                                         &rad, c.ext_rad[(size_t)(doy - 1) * c.nrow + c.ext_row[s]]);
     } else {
-      vertical_cell<R>(c, s, gam, canopy, soil, gsnow, st.snow_band + i, N, days, status, psum, laf, laf,
+      vertical_cell<R, false, true>(c, s, gam, canopy, soil, gsnow, st.snow_band + i, N, days, status, psum, laf, laf,
                        R(f.prec[fo]) * pf, Tf, pet, o);
     }
     const size_t ri = ring_row(ring, d) * N + i;
@@ -644,14 +644,17 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
               const size_t ui = (size_t)c.up_idx[k] * M + mm;
               // an upstream cell of the same unit was routed this step, earlier in this loop
               const double qu = (GL && unit >= 0 && wu.unit_of[c.up_idx[k]] == unit)
-                                    ? q_now[ui] : upstream_value<!FUSED>(sync, q_prev + ui, failed);
+                                    ? q_now[ui]
+                                    : ENS ? __ldcg(q_prev + ui) : upstream_value<!FUSED>(sync, q_prev + ui, failed);
               up += qu;
               if constexpr (WT)   // the energy the inflow carries (calcWaterTemp.cpp:76-83)
                 e_up += qu * WT_RC * (upstream_value<!FUSED>(sync, t_prev0 + (size_t)kk * N + ui, failed) + WT_CONV_K);
             }
             return up;
           };
-          if constexpr (WT) inflow_up();   // the water temperature's day begins with it
+          // the water temperature's day begins with the inflow; an ensemble's 64
+          // registers hold it rather than the routing state before it
+          if constexpr (WT || ENS) inflow_up();
           RState<R> rs = load_rstate(st, si, fl);
           RTerms<R> rt;
           // the water temperature (routing.cpp:4241-4513) body by body inside
@@ -680,16 +683,17 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
             // storages stay, nothing flows on, and the inflow stays behind in
             // G_riverInflow, i.e. leaves the system (a negative leak: the leak
             // counts water the model adds)
-            if constexpr (!WT) inflow_up();
+            if constexpr (!WT && !ENS) inflow_up();
             tv = R(0);
             rt.p_ow = R(0); rt.e_ow = R(0); rt.leak = R(-up); rt.velocity = R(0);
           } else {
             tv = routing_cell<R, WT, WU, GL, RO>(c, s, rs, doy, month, laf, laf_prev, o,
-                                                 [&]() { return WT ? up : inflow_up(); }, rt, &wtd, &wu, wrow, si, N, &ro);
+                                                 [&]() { return WT || ENS ? up : inflow_up(); }, rt, &wtd, &wu, wrow, si, N, &ro);
             if (!FUSED && failed) return;
             store_rstate(st, si, rs, fl);
           }
-          st_outflow(q_now + si, (double)tv);
+          if (ENS) q_now[si] = (double)tv;
+          else st_outflow(q_now + si, (double)tv);
           if constexpr (WT) {
             // a cell without continental area keeps the reference's initial 15 degrees (routing.cpp:174)
             const double tr = nocont ? 15. : wtd.river((double)rs.river, (double)c.bw[s], (double)c.rlen[s],

@@ -69,12 +69,21 @@ template <> struct E<double> {
   static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
   static __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
   static __device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
+  // a / b correctly rounded from the correctly rounded reciprocal y of b: the quotient
+  // a y, within an ulp, corrected by its exact remainder (P. Markstein, "IA-64 and
+  // Elementary Functions", 2000, ch. 8) -- three operations where the general division
+  // takes about ten
+  static __device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    return fma(fma(-q, b, a), y, q);
+  }
 };
 template <> struct E<float> {
   static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
   static __device__ __forceinline__ float add(float a, float b) { return a + b; }
   static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
   static __device__ __forceinline__ float div(float a, float b) { return a / b; }
+  static __device__ __forceinline__ float div_by(float a, float b, float) { return a / b; }
 };
 
 // Comparisons of the day step's hot loops.  On GB300 a double compare issues on
@@ -105,11 +114,28 @@ template <> struct C<double> {
   }
   static __device__ __forceinline__ bool is_zero(double a) { return (__double_as_longlong(a) << 1) == 0; }
   static __device__ __forceinline__ bool is_one(double a) { return __double_as_longlong(a) == 0x3FF0000000000000ll; }
+  static __device__ __forceinline__ bool equal(double a, double b) { return key(a) == key(b); }
+};
+// The same for the water bodies, whose storages keep a NaN where the inputs bring one:
+// false with a NaN on either side, as the FP64 compares are (a NaN that arithmetic
+// left has its quiet bit, the top one of the fraction, set).
+template <class R> struct Cn;
+template <> struct Cn<double> {
+  typedef C<double> c;
+  static __device__ __forceinline__ bool nan(double a) { return ((uint32_t)__double2hiint(a) << 1) > 0xffe00000u; }
+  static __device__ __forceinline__ bool gt(double a, double b) { return c::gt(a, b) && !nan(a) && !nan(b); }
+  static __device__ __forceinline__ bool ge(double a, double b) { return c::le(b, a) && !nan(a) && !nan(b); }
+  static __device__ __forceinline__ bool lt0(double a) { return c::lt0(a) && !nan(a); }
+  static __device__ __forceinline__ bool gt0(double a) { return c::gt0(a) && !nan(a); }
+  static __device__ __forceinline__ bool le0(double a) { return c::le0(a) && !nan(a); }
+  static __device__ __forceinline__ bool gt_c(double a, double k) { return c::gt_c(a, k) && !nan(a); }
+  static __device__ __forceinline__ bool abs_le_c(double a, double k) { return c::abs_le_c(a, k); }
 };
 template <> struct C<float> {
   static __device__ __forceinline__ bool gt(float a, float b) { return a > b; }
   static __device__ __forceinline__ bool le(float a, float b) { return a <= b; }
   static __device__ __forceinline__ bool lt(float a, float b) { return a < b; }
+  static __device__ __forceinline__ bool ge(float a, float b) { return a >= b; }
   static __device__ __forceinline__ bool lt0(float a) { return a < 0.f; }
   static __device__ __forceinline__ bool gt0(float a) { return a > 0.f; }
   static __device__ __forceinline__ bool le0(float a) { return a <= 0.f; }
@@ -118,6 +144,31 @@ template <> struct C<float> {
   static __device__ __forceinline__ bool abs_le_c(float a, float c) { return fabsf(a) <= c; }
   static __device__ __forceinline__ bool is_zero(float a) { return a == 0.f; }
   static __device__ __forceinline__ bool is_one(float a) { return a == 1.f; }
+  static __device__ __forceinline__ bool equal(float a, float b) { return a == b; }
+};
+template <> struct Cn<float> : C<float> {};
+
+// Operations of branches that hardly any cell takes.  The compiler turns a short
+// branch into predicated instructions, and an FP64 instruction that no lane executes
+// holds the pipe like one that all execute (measured 68 cycles per warp against 11
+// for the branch around a call); so in FP64 these are calls.  FP32: the plain
+// operations.
+template <class R> struct Rare;
+__device__ __noinline__ double rare_mul(double a, double b) { return a * b; }
+__device__ __noinline__ double rare_add(double a, double b) { return a + b; }
+__device__ __noinline__ double rare_sub(double a, double b) { return a - b; }
+__device__ __noinline__ double rare_fma(double a, double b, double c) { return fma(a, b, c); }
+template <> struct Rare<double> {
+  static __device__ __forceinline__ double mul(double a, double b) { return rare_mul(a, b); }
+  static __device__ __forceinline__ double add(double a, double b) { return rare_add(a, b); }
+  static __device__ __forceinline__ double sub(double a, double b) { return rare_sub(a, b); }
+  static __device__ __forceinline__ double muladd(double a, double b, double c) { return rare_fma(a, b, c); }
+};
+template <> struct Rare<float> {
+  static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
+  static __device__ __forceinline__ float add(float a, float b) { return a + b; }
+  static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
+  static __device__ __forceinline__ float muladd(float a, float b, float c) { return a * b + c; }
 };
 
 template <class R>
@@ -301,9 +352,10 @@ __device__ __forceinline__ Pet<R> pet_of(const DevCellsT<R> &c, int s, const Rad
 //   band        : the cell's snow bands, band[e * bstride]
 //   Pin         : precipitation (times a member's factor in an ensemble)
 //   pet         : the day's potential evapotranspiration
+//   SAME        : the land fraction is the day before's (prevLAF == landAreaFrac)
 //   OUT, vs     : the output grids (monthly and daily) of the cell-day, which take
 //                 its radiation terms rad and ext_rad too
-template <class R, bool OUT = false>
+template <class R, bool OUT = false, bool SAME = false>
 __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R gamma_soil, R &canopy, R &soil,
                                               R &gsnow, R *band, size_t bstride, int &days, int &status, R &psum,
                                               R landAreaFrac, R prevLAF, R Pin, float Tf, const Pet<R> &pet, VOut<R> &o,
@@ -407,8 +459,8 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
   const bool land = cmp::gt0(landAreaFrac);
   // prevLAF / landAreaFrac; exactly 1 while the land fraction does not change, and
   // then the storages are not rescaled (x * 1 = x)
-  const R ratio = !land ? R(0) : (prevLAF == landAreaFrac ? R(1) : prevLAF / landAreaFrac);
-  const bool rescale = !cmp::is_one(ratio);
+  const R ratio = !land ? R(0) : (SAME || cmp::equal(prevLAF, landAreaFrac) ? R(1) : prevLAF / landAreaFrac);
+  const bool rescale = !SAME && !cmp::is_one(ratio);
   // the correction factor is 1 in most cells: its products and the storage change
   // they weigh (the same bits: x * 1 = x, y * 0 + x * 1 = x) are left out there
   const bool corrected = !cmp::is_one(cfa);
@@ -435,19 +487,15 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
       }
       const R cwc = canopy;
       canopyEvapo = dailyPET * m::pow(cwc * m::rcp(maxcs), R(0.66666666));   // maxcs > 1e-5 mcwh
-      if (cmp::gt(canopyEvapo, cwc)) {
-        canopyEvapo = cwc;
-        soilPET = dailyPET - cwc;
-        canopy = R(0);
-      } else {
-        canopy -= canopyEvapo;
-        soilPET = dailyPET - canopyEvapo;
-      }
+      const bool dry = cmp::gt(canopyEvapo, cwc);
+      if (dry) canopyEvapo = cwc;
+      soilPET = dailyPET - canopyEvapo;
+      canopy = dry ? R(0) : canopy - canopyEvapo;
     } else {
       prec_to_soil = dailyPrec;
       soilPET = dailyPET;
     }
-    if (corrected) lsc += canopy - initialStorage;
+    if (corrected) lsc = Rare<R>::add(lsc, Rare<R>::sub(canopy, initialStorage));
   }
   if (cmp::lt0(soilPET)) soilPET = R(0);
   if constexpr (OUT) {
@@ -551,7 +599,7 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
           sb -= melt;
         }
       }
-      if (corrected) snowChange += sb - initialStorage;
+      if (corrected) snowChange = Rare<R>::add(snowChange, Rare<R>::sub(sb, initialStorage));
       if (e == 0) above0 = !snowfall;
       gs += sb;
       if constexpr (fp32) effPrec += effBefore + melt;
@@ -578,7 +626,7 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
         if (n_evap) snowEvapo = fma((double)n_evap, soilPET, snowEvapo);
       }
       snowEvapo *= invB;
-      if (corrected) lsc += snowChange * invB;
+      if (corrected) lsc = Rare<R>::muladd(snowChange, invB, lsc);
     }
   }
   gsnow = gs;
@@ -623,7 +671,7 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
     if (rescale) soil *= ratio;
     initialStorage = soil;
     if (cmp::gt(soil, Smax)) {
-      overflow = soil - Smax;
+      overflow = Rare<R>::sub(soil, Smax);
       soil = Smax;
     }
     if (above0) {
@@ -636,12 +684,12 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
         if (cmp::abs_le_c(soil, R(WG_MIN_STOR_VOL))) soil = R(0);
         effPrec = R(0);
         if (cmp::lt0(soil)) {
-          dailyAET += soil;
+          dailyAET = Rare<R>::add(dailyAET, soil);
           soil = R(0);
         }
         if (corrected) {
-          runoff *= cfa;
-          immediate *= cfa;
+          runoff = Rare<R>::mul(runoff, cfa);
+          immediate = Rare<R>::mul(immediate, cfa);
         }
         const R fgr = c.fg[s] * runoff;
         gwr = cmp::lt(c.rgmax[s], fgr) ? c.rgmax[s] : fgr;
@@ -654,28 +702,28 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
           soil += pot * c.inv_cfa[s];
         }
         if (cmp::gt(soil, Smax)) {
-          overflow += soil - Smax;
+          overflow = Rare<R>::add(overflow, Rare<R>::sub(soil, Smax));
           soil = Smax;
         }
-        if (corrected) overflow *= cfa;
+        if (corrected) overflow = Rare<R>::mul(overflow, cfa);
         total = runoff;
         if (!cmp::is_zero(immediate)) total += immediate;
-        if (!cmp::is_zero(overflow)) total += overflow;
+        if (!cmp::is_zero(overflow)) total = Rare<R>::add(total, overflow);
       }
     } else {
       if (corrected) {
-        overflow *= cfa;
-        effPrec *= cfa;
+        overflow = Rare<R>::mul(overflow, cfa);
+        effPrec = Rare<R>::mul(effPrec, cfa);
       }
-      total += overflow + effPrec;
+      total = overflow + effPrec;
       dailyAET = R(0);
-      leak -= cfa * immediate;   // built-up runoff is dropped in this branch
+      if (!cmp::is_zero(immediate)) leak = Rare<R>::sub(leak, Rare<R>::mul(cfa, immediate));   // built-up runoff is dropped in this branch
     }
     gwr_route = gwr;   // G_dailyGwRecharge (daily.cpp:1232)
     cellAET = dailyAET + canopyEvapo + snowEvapo;
     if (corrected) {
-      lsc += soil - initialStorage;
-      cellAET = (lsc - dailyPrec) * (cfa - R(1.0)) + cellAET * cfa;
+      lsc = Rare<R>::add(lsc, Rare<R>::sub(soil, initialStorage));
+      cellAET = Rare<R>::muladd(Rare<R>::sub(lsc, dailyPrec), Rare<R>::sub(cfa, R(1.0)), Rare<R>::mul(cellAET, cfa));
     }
     if (cmp::lt0(cellAET)) {
       neg_land_aet = cellAET;
@@ -683,16 +731,17 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
     }
   }
   // surface runoff (daily.cpp:1244-1257)
-  if (cmp::lt0(neg_land_aet)) total = total + neg_land_aet;
+  if (cmp::lt0(neg_land_aet)) total = Rare<R>::add(total, neg_land_aet);
   if (cmp::lt0(total)) {
-    leak -= total;
+    leak = Rare<R>::sub(leak, total);
     total = R(0);
   }
-  if (cmp::lt0(total - gwr)) {
-    soil += total - gwr;
-    gwr = total;
-  }
   o.rs = total - gwr;
+  if (cmp::lt0(o.rs)) {
+    soil = Rare<R>::add(soil, o.rs);
+    gwr = total;
+    o.rs = R(0);
+  }
   o.gwr = gwr_route;
   o.transfer = transfer;
   o.land_in = dailyPrec;
@@ -773,7 +822,7 @@ __device__ __forceinline__ R river_velocity(const DevCellsT<R> &c, int s, R rive
   const R wp = bw + R(2.0 * 2.23606797749979) * depth;   // 2 sqrt(5)
   const R hr = csa * m::rcp(wp);
   const R v = c.inv_mr[s] * m::pow(hr, R(2. / 3.)) * c.sqrt_slope[s] * R(86.4);
-  return (v < R(0.00001)) ? R(0.00001) : v;
+  return C<R>::lt_c(v, R(0.00001)) ? R(0.00001) : v;
 }
 
 // routingClass::updateNetAbstractionGW (routing.cpp:5503-5572): the day's net
@@ -885,7 +934,8 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
   }
   const R f_land = c.area_f[s] * laf;
   typedef C<R> cmp;
-  R dlsr = cmp::le0(laf) ? v.transfer * c.area_f[s] * laf_prev : v.rs * f_land;
+  R dlsr = v.rs * f_land;
+  if (cmp::le0(laf)) dlsr = Rare<R>::mul(Rare<R>::mul(v.transfer, c.area_f[s]), laf_prev);
   // groundwater (routing.cpp:2061-2200)
   const R gw0 = st.gw;
   R netGWin = v.gwr * f_land;
@@ -942,18 +992,19 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
   R outflow = R(0);
   const R a6 = c.a6[s];
 
+  typedef Cn<R> cn;
   if (fl & F_LOCLAKE) {  // local lake (routing.cpp:2318-2490)
     const R S0 = st.loclake, maxS = c.maxs_ll[s], rf = st.rf_loclake;
     R evapo = (R(1.0) - cfa) * owp * rf + cfa * owpet * rf;
-    if (evapo < R(0)) evapo = R(0);
+    if (cn::lt0(evapo)) evapo = R(0);
     const R pin = owp * rf * a6 * c.ll100[s];
     const R TI = inflow + pin;
     const R PETgwr = evapo * a6 * c.ll100[s];
     R PETgwrMax = S0 + maxS + TI;
     const R avail = PETgwrMax;
-    if (PETgwrMax < R(0)) PETgwrMax = R(0);
+    if (cn::lt0(PETgwrMax)) PETgwrMax = R(0);
     R S;
-    if (PETgwr > PETgwrMax) {
+    if (cn::gt(PETgwr, PETgwrMax)) {
       S = -maxS;
       rt.e_ow += avail;
       if constexpr (WT || RO) evapo *= PETgwrMax / PETgwr;   // routing.cpp:2400-2404
@@ -962,14 +1013,14 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       rt.e_ow += PETgwr;
     }
     rt.p_ow += pin;
-    if (S0 > R(0)) {
+    if (cn::gt0(S0)) {
       outflow = c.sw_k[s] * S0 * m::pow(S0 * c.inv_maxs_ll[s], R(1.5));
-      if (S <= R(0)) outflow = R(0);
-      else if (outflow > S) outflow = S;
+      if (cn::le0(S)) outflow = R(0);
+      else if (cn::gt(outflow, S)) outflow = S;
     } else outflow = R(0);
     S -= outflow;
-    if (m::fabs_(S) <= R(WG_MIN_STOR_VOL)) S = R(0);
-    if (S > maxS) {
+    if (cn::abs_le_c(S, R(WG_MIN_STOR_VOL))) S = R(0);
+    if (cn::gt(S, maxS)) {
       outflow += S - maxS;
       S = maxS;
     }
@@ -978,18 +1029,18 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     if constexpr (RO) ro->owe += (double)evapo * (double)a6 * (double)c.ll100[s];
     R r = R(1.) - m::pow(m::fabs_(S - maxS) * (R(0.5) * c.inv_maxs_ll[s]), c.evx[s]);
     st.loclake = S;
-    st.rf_loclake = r < R(0) ? R(0) : (r > R(1) ? R(1) : r);
+    st.rf_loclake = cn::lt0(r) ? R(0) : (cn::gt_c(r, R(1)) ? R(1) : r);
   }
   if (fl & F_LOCWETL) {  // local wetland (routing.cpp:2495-2617)
     const R S0 = st.locwetl, maxS = c.maxs_lw[s], rf = st.rf_locwetl;
     R evapo = (R(1.0) - cfa) * owp * rf + cfa * owpet * rf;
-    if (evapo < R(0)) evapo = R(0);
+    if (cn::lt0(evapo)) evapo = R(0);
     const R pin = owp * rf * a6 * c.lw100[s];
     const R TI = inflow + pin;
     const R PETgwr = evapo * a6 * c.lw100[s];
     const R PETgwrMax = S0 + TI;
     R S;
-    if (PETgwr > PETgwrMax) {
+    if (cn::gt(PETgwr, PETgwrMax)) {
       S = R(0);
       rt.e_ow += PETgwrMax;
       if constexpr (WT || RO) evapo *= PETgwrMax / PETgwr;
@@ -998,13 +1049,13 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       rt.e_ow += PETgwr;
     }
     rt.p_ow += pin;
-    if (m::fabs_(S) <= R(WG_MIN_STOR_VOL)) S = R(0);
-    if (S > R(0)) {
+    if (cn::abs_le_c(S, R(WG_MIN_STOR_VOL))) S = R(0);
+    if (cn::gt0(S)) {
       outflow = c.sw_k[s] * S * m::pow(S * c.inv_maxs_lw[s], R(2.5));
-      if (outflow > S) outflow = S;
+      if (cn::gt(outflow, S)) outflow = S;
     } else outflow = R(0);
     S -= outflow;
-    if (S > maxS) {
+    if (cn::gt(S, maxS)) {
       outflow += S - maxS;
       S = maxS;
     }
@@ -1016,14 +1067,14 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     }
     R r = R(1.) - m::pow(m::fabs_(S - maxS) * c.inv_maxs_lw[s], c.evx[s]);
     st.locwetl = S;
-    st.rf_locwetl = r < R(0) ? R(0) : (r > R(1) ? R(1) : r);
+    st.rf_locwetl = cn::lt0(r) ? R(0) : (cn::gt_c(r, R(1)) ? R(1) : r);
   }
   inflow = R((double)inflow + inflow_up());   // routing.cpp:2623-2624
   if constexpr (WT) wtd->locals_done();
   if (fl & F_GLOLAKE) {  // global lake (routing.cpp:2630-2804)
     const R S0 = st.glolake, maxS = c.maxs_gl[s], rf = st.rf_glolake;
     R evapo = (R(1.0) - cfa) * owp + cfa * owpet * rf;
-    if (evapo < R(0)) evapo = R(0);
+    if (cn::lt0(evapo)) evapo = R(0);
     const R pin = owp * c.la6[s];
     const R TI = inflow + pin;
     R PU = evapo * c.la6[s];
@@ -1036,7 +1087,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     const R PUmax = TI + maxS + S0;
     rt.p_ow += pin;
     R S;
-    if (PU > PUmax) {
+    if (cn::gt(PU, PUmax)) {
       S = -maxS;
       outflow = R(0);
       rt.e_ow += PUmax;
@@ -1046,17 +1097,17 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       if constexpr (WU) remUseGL = R(0);
       S = S0 * c.sw_e[s] + c.sw_ik[s] * (TI - PU) * c.sw_ome[s];
       outflow = TI + S0 - S - PU;
-      if (S > maxS) {
+      if (cn::gt(S, maxS)) {
         outflow += S - maxS;
         S = maxS;
       }
-      if (outflow < R(0)) {
+      if (cn::lt0(outflow)) {
         outflow = R(0);
         S = S0 + TI - PU;
       }
       rt.e_ow += PU;
     }
-    if (m::fabs_(S) <= R(WG_MIN_STOR_VOL)) S = R(0);
+    if (cn::abs_le_c(S, R(WG_MIN_STOR_VOL))) S = R(0);
     inflow = outflow;
     if constexpr (WU) dailyActualUse = remGL0 - remUseGL;   // routing.cpp:2788
     if constexpr (WT) wtd->glolake((double)S0 + (double)maxS, evapo, outflow);
@@ -1066,13 +1117,13 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     }
     R r = R(1.) - m::pow(m::fabs_(S - maxS) * (R(0.5) * c.inv_maxs_gl[s]), c.evx[s]);
     st.glolake = S;
-    st.rf_glolake = r < R(0) ? R(0) : (r > R(1) ? R(1) : r);
+    st.rf_glolake = cn::lt0(r) ? R(0) : (cn::gt_c(r, R(1)) ? R(1) : r);
   }
   if (fl & F_RES) {  // reservoir (routing.cpp:2807-3082), each expression rounded as the reference rounds it
     typedef E<R> x;
     const R S0 = st.res, maxS = c.rcap[s], rf = st.rf_res;
     R evapo = x::add(x::mul(x::sub(R(1.0), cfa), owp), x::mul(cfa, x::mul(owpet, rf)));   // routing.cpp:2832-2836
-    if (evapo < R(0)) evapo = R(0);
+    if (cn::lt0(evapo)) evapo = R(0);
     const R pin = x::mul(owp, c.ra6[s]);
     const R TI = x::add(inflow, pin);
     const R PETgwr = x::mul(evapo, c.ra6[s]);
@@ -1088,7 +1139,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       ro->res_in = (double)inflow;
       ro->p_lake += (double)pin;
     }
-    if (PETgwr > PETgwrMax) {
+    if (cn::gt(PETgwr, PETgwrMax)) {
       S = S0 + TI - PETgwrMax;
       rt.e_ow += PETgwrMax;
       if constexpr (WT || RO) evapo *= PETgwrMax / PETgwr;
@@ -1115,7 +1166,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
         }
       }
     }
-    if (m::fabs_(S) <= R(WG_MIN_STOR_VOL)) S = R(0);
+    if (cn::abs_le_c(S, R(WG_MIN_STOR_VOL))) S = R(0);
     R K = st.k_release;
     if (month == c.start_month[s] - 1 && doy == c_first_day_in_month[month]) {
       K = (S < c.rcap01[s]) ? R(0.1) : x::div(S, x::mul(maxS, R(0.85)));   // routing.cpp:2959-2962
@@ -1127,17 +1178,17 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     if (c.c_ratio[s] >= R(0.5)) release = x::mul(K, prov);
     else
       release = x::add(x::mul(x::mul(c.c4[s], K), prov),
-                       x::div(x::mul(x::mul(c.one_m_c4[s], inflow), R(1.0e9)), R(86400.)));
+                       x::div_by(x::mul(x::mul(c.one_m_c4[s], inflow), R(1.0e9)), R(86400.), R(1. / 86400.)));
     // km3 per day; a tenth below 10 % of the capacity (routing.cpp:3012-3017)
-    outflow = (S >= c.rcap01[s]) ? x::div(x::mul(release, R(86400.)), R(1.0e9))
-                                 : x::div(x::mul(x::mul(R(0.1), release), R(86400.)), R(1.0e9));
-    if (outflow < R(0)) outflow = R(0);
+    outflow = cn::ge(S, c.rcap01[s]) ? x::div_by(x::mul(release, R(86400.)), R(1.0e9), R(1. / 1.0e9))
+                                 : x::div_by(x::mul(x::mul(R(0.1), release), R(86400.)), R(1.0e9), R(1. / 1.0e9));
+    if (cn::lt0(outflow)) outflow = R(0);
     S -= outflow;
-    if (S > maxS) {
+    if (cn::gt(S, maxS)) {
       outflow += S - maxS;
       S = maxS;
     }
-    if (S < R(0)) {
+    if (cn::lt0(S)) {
       outflow += S;
       S = R(0);
     }
@@ -1148,9 +1199,10 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       ro->owe += (double)evapo * (double)c.ra6[s];
       ro->res_out = (double)outflow;
     }
-    R r = R(1.) - m::pow(x::div(m::fabs_(S - maxS), maxS), R(2.81383));   // routing.cpp:3071-3072
+    R r = R(1.) - m::pow(cn::gt0(maxS) ? x::div_by(m::fabs_(S - maxS), maxS, c.inv_rcap[s])
+                                          : x::div(m::fabs_(S - maxS), maxS), R(2.81383));   // routing.cpp:3071-3072
     st.res = S;
-    st.rf_res = r < R(0) ? R(0) : (r > R(1) ? R(1) : r);
+    st.rf_res = cn::lt0(r) ? R(0) : (cn::gt_c(r, R(1)) ? R(1) : r);
   }
   if constexpr (WU) {   // routing.cpp:3083-3172
     if (fl & (F_RES | F_GLOLAKE)) {
@@ -1198,14 +1250,14 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
   if (fl & F_GLOWETL) {  // global wetland (routing.cpp:3178-3297)
     const R S0 = st.glowetl, maxS = c.maxs_gw[s], rf = st.rf_glowetl;
     R evapo = (R(1.0) - cfa) * owp * rf + cfa * owpet * rf;
-    if (evapo < R(0)) evapo = R(0);
+    if (cn::lt0(evapo)) evapo = R(0);
     const R pin = owp * rf * a6 * c.gw100[s];
     const R TI = inflow + pin;
     const R PETgwr = evapo * a6 * c.gw100[s];
     const R PETgwrMax = TI + S0;
     rt.p_ow += pin;
     R S;
-    if (PETgwr > PETgwrMax) {
+    if (cn::gt(PETgwr, PETgwrMax)) {
       S = R(0);
       outflow = R(0);
       rt.e_ow += PETgwrMax;
@@ -1215,11 +1267,11 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       outflow = TI + S0 - S - PETgwr;
       rt.e_ow += PETgwr;
     }
-    if (S > maxS) {
+    if (cn::gt(S, maxS)) {
       outflow += S - maxS;
       S = maxS;
     }
-    if (m::fabs_(S) <= R(WG_MIN_STOR_VOL)) S = R(0);
+    if (cn::abs_le_c(S, R(WG_MIN_STOR_VOL))) S = R(0);
     inflow = outflow;
     if constexpr (WT) wtd->glowetl(S0, evapo, rf, outflow);
     if constexpr (RO) {   // routing.cpp:3194-3210
@@ -1228,7 +1280,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     }
     R r = R(1.) - m::pow(m::fabs_(S - maxS) * c.inv_maxs_gw[s], c.evx[s]);
     st.glowetl = S;
-    st.rf_glowetl = r < R(0) ? R(0) : (r > R(1) ? R(1) : r);
+    st.rf_glowetl = cn::lt0(r) ? R(0) : (cn::gt_c(r, R(1)) ? R(1) : r);
   }
   // river (routing.cpp:3385-3514)
   if (c.frac_routing && !(fl & F_SINK)) {   // routing.cpp:3408-3412
@@ -1258,7 +1310,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
       remainingUse = R(0);
     }
   } else if ((cmp::lt0(inflow) || cmp::lt0(S0)) &&
-             cmp::lt0(inflow * omeK + K * S0 * eK)) {   // sign of RivEvapoRemUseMax (routing.cpp:3444-3449)
+             cmp::lt0(Rare<R>::muladd(inflow, omeK, Rare<R>::mul(Rare<R>::mul(K, S0), eK)))) {   // sign of RivEvapoRemUseMax (routing.cpp:3444-3449)
     const R maxUse = inflow + K * S0 * eK * m::rcp(omeK);   // K >= 1e-5 / length: omeK > 0
     S = R(0);
     transported = inflow + S0 - maxUse;
@@ -1268,7 +1320,7 @@ __device__ __forceinline__ R routing_cell(const DevCellsT<R> &c, int s, RState<R
     transported = inflow + S0 - S;
   }
   if (cmp::lt0(transported)) {
-    rt.leak -= transported;
+    rt.leak = Rare<R>::sub(rt.leak, transported);
     transported = R(0);
   }
   st.river = S;
