@@ -62,7 +62,14 @@ __device__ __forceinline__ u64 exp2_mant(u64 f) {
   return t + mul_hi(t, mul_hi(r, a1));
 }
 
-// 2^(n + f), f in units of 2^-64, rounded to a double
+// 2^(n + f), f in units of 2^-64, rounded to a double; n within the exponents of
+// normal doubles
+__device__ __forceinline__ double exp2_normal(int n, u64 f) {
+  const u64 u = exp2_mant(f);
+  return double_of((u >> 11) + (((u64)((uint32_t)(n + 1022) << 20) << 32) | ((lo32(u) >> 10) & 1u)));
+}
+
+// the same for any n
 __device__ __forceinline__ double exp2_fixed(int n, u64 f) {
   const u64 u = exp2_mant(f);
   if ((unsigned)(n + 1021) >= 2045u) {                       // subnormal, zero or infinite
@@ -75,30 +82,34 @@ __device__ __forceinline__ double exp2_fixed(int n, u64 f) {
   return double_of((u >> 11) + (((u64)((uint32_t)(n + 1022) << 20) << 32) | ((lo32(u) >> 10) & 1u)));
 }
 
+// exp of an argument of 32 or more, or not a number: out of line, since the hot path
+// never has one and a branch that holds no code of its own costs least
+__device__ __noinline__ double exp_any(double x) {
+  const u64 b = bits_of(x), log2e = 0xb8aa3b295c17f0bcull;   // units of 2^-63
+  const int e = (int)((hi32(b) >> 20) & 0x7ff) - 1023;
+  if (e >= 10) {                                             // beyond the range of a double
+    if ((b << 1) > 0xffe0000000000000ull) return x;          // NaN
+    return (i64)b < 0 ? 0. : double_of(0x7ff0000000000000ull);
+  }
+  const u64 m = (b << 11) | 0x8000000000000000ull;           // |x| = m 2^(e - 63)
+  const u64 p = __umul64hi(m, log2e);
+  const uint32_t s = (uint32_t)((int)hi32(b) >> 31);         // -(n + f) = ~n + ~f
+  return exp2_fixed((int)((uint32_t)(p >> (62 - e)) ^ s),
+                    ((p << (e + 2)) | ((m * log2e) >> (62 - e))) ^ (u64)(i64)(int)s);
+}
+
 __device__ __forceinline__ double exp(double x) {
   const u64 b = bits_of(x);
   const int e = (int)((hi32(b) >> 20) & 0x7ff) - 1023;
-  const u64 m = (b << 11) | 0x8000000000000000ull;           // |x| = m 2^(e - 63)
-  const u64 log2e = 0xb8aa3b295c17f0bcull;                   // units of 2^-63
-  u64 p = mul_hi(m, log2e);                                  // |x| log2 e = p 2^(e - 62)
-  uint32_t n;
-  u64 f;
-  if (e < 5) {                                               // |x| < 32: every argument of the hot path
-    p >>= min(max(-2 - e, 0), 63);
-    const int k = max(e + 2, 0);
-    n = __funnelshift_l(hi32(p), 0u, k);
-    f = ((u64)__funnelshift_l(lo32(p), hi32(p), k) << 32) | (lo32(p) << k);
-  } else {
-    if (e >= 10) {                                           // beyond the range of a double
-      if ((b << 1) > 0xffe0000000000000ull) return x;        // NaN
-      return (i64)b < 0 ? 0. : double_of(0x7ff0000000000000ull);
-    }
-    p = __umul64hi(m, log2e);
-    n = (uint32_t)(p >> (62 - e));
-    f = (p << (e + 2)) | ((m * log2e) >> (62 - e));
-  }
+  if (e >= 5) return exp_any(x);
+  const u64 m = (b << 11) | 0x8000000000000000ull;           // |x| = m 2^(e - 63), below 32
+  u64 p = mul_hi(m, 0xb8aa3b295c17f0bcull);                  // |x| log2 e = p 2^(e - 62)
+  p >>= min(max(-2 - e, 0), 63);
+  const int k = max(e + 2, 0);
   const uint32_t s = (uint32_t)((int)hi32(b) >> 31);         // -(n + f) = ~n + ~f
-  return exp2_fixed((int)(n ^ s), f ^ (u64)(i64)(int)s);
+  const uint32_t n = __funnelshift_l(hi32(p), 0u, k) ^ s;
+  const u64 f = (((u64)__funnelshift_l(lo32(p), hi32(p), k) << 32) | (lo32(p) << k)) ^ (u64)(i64)(int)s;
+  return exp2_normal((int)n, f);
 }
 
 // exp(-x) for x >= 0 where the caller goes on with 1 - exp(-x), as the river's
@@ -160,7 +171,8 @@ __device__ __forceinline__ double log(double x) {
   return (double)l * double_of((u64)(959 + sh) << 52) * 0.6931471805599453;   // 2^(sh - 64)
 }
 
-__device__ __forceinline__ double pow(double x, double y) {
+// x^y for any x and y
+__device__ __noinline__ double pow_any(double x, double y) {
   const u64 b = bits_of(x), yb = bits_of(y);
   if ((i64)b <= 0) return 0.0;                               // x <= 0 (and -0)
   if (b == 0x3ff0000000000000ull) return 1.0;                // x == 1
@@ -191,6 +203,25 @@ __device__ __forceinline__ double pow(double x, double y) {
   return exp2_fixed((int)(n ^ s), f ^ (u64)(i64)(int)s);
 }
 
+// x^y: the integer part of y log2 x in k bits of the product, 1 <= k <= 31, and the
+// result a normal double, else pow_any; x <= 0 gives 0
+__device__ __forceinline__ double pow(double x, double y) {
+  const u64 b = bits_of(x), yb = bits_of(y);
+  int sh;
+  const i64 l = log2_fixed(b, sh);
+  const uint32_t ls = (uint32_t)((int)hi32((u64)l) >> 31);
+  const u64 la = ((u64)l ^ (u64)(i64)(int)ls) - (u64)(i64)(int)ls;
+  const int k = sh + (int)((hi32(yb) >> 20) & 0x7ff) - 1022;
+  const u64 p = mul_hi(la, (yb << 11) | 0x8000000000000000ull);
+  const uint32_t s = ls ^ (uint32_t)((int)hi32(yb) >> 31);
+  const uint32_t n = (hi32(p) >> ((32 - k) & 31)) ^ s;
+  const u64 f = (((u64)__funnelshift_l(lo32(p), hi32(p), k) << 32) | (lo32(p) << (k & 31))) ^ (u64)(i64)(int)s;
+  // x positive and not a normal number, or a format or result outside the above
+  if ((i64)b > 0 && (hi32(b) - 0x00100000u >= 0x7fe00000u || (unsigned)(k - 1) >= 31u || n + 1000u > 2000u))
+    return pow_any(x, y);
+  return (i64)b <= 0 ? 0. : exp2_normal((int)n, f);
+}
+
 // 1/(m 2^-63) for m in [2^63, 2^64), in units of 2^-64: the single-precision
 // hardware reciprocal r of the leading 24 bits, lowered so that e = 1 - m r is
 // positive (below 2^-20), then r (1 + e + e^2)
@@ -216,6 +247,47 @@ __device__ __forceinline__ double rcp_pos(double x) {
   // zero, subnormal, infinite and NaN arguments give NaN, those from 2^1022 on 0
   if (ex - 1u >= 2044u) return double_of(ex - 1u >= 2046u ? 0x7ff8000000000000ull : 0ull);
   return v;
+}
+
+__device__ __noinline__ double div_any(double a, double b) { return a / b; }
+
+// a / b to half an ulp and 2^-8 more for normal a and b with a normal quotient (a = 0
+// gives 0 with the quotient's sign), anything else through the general division
+__device__ __forceinline__ double div(double a, double b) {
+  const u64 ab = bits_of(a), bb = bits_of(b);
+  const int ea = (int)((hi32(ab) >> 20) & 0x7ff), eb = (int)((hi32(bb) >> 20) & 0x7ff);
+  const u64 sign = (ab ^ bb) & 0x8000000000000000ull;
+  u64 q = mul_hi((ab << 11) | 0x8000000000000000ull, rcp_mant((bb << 11) | 0x8000000000000000ull));
+  const uint32_t low = (hi32(q) >> 31) ^ 1u;                 // the quotient of the mantissas is below 1
+  q <<= low;
+  const int e = ea - eb + 1022 - (int)low;                   // biased exponent less one
+  const double r = double_of(((q >> 11) + (((u64)((uint32_t)e << 20) << 32) | ((lo32(q) >> 10) & 1u))) | sign);
+  if ((unsigned)(eb - 1) >= 2046u || ((unsigned)(ea - 1) >= 2046u && (ab << 1) != 0) || (ea && (unsigned)(e - 1) >= 2043u))
+    return div_any(a, b);
+  return ea ? r : double_of(sign);
+}
+
+__device__ __noinline__ double sqrt_any(double x) { return ::sqrt(x); }
+
+// square root of a positive normal number to half an ulp and 2^-8 more: m in [1/4, 1),
+// the single-precision reciprocal root y of its leading bits, e = 1 - m y^2, then
+// m y (1 + e/2 + 3 e^2/8) (Markstein 2000, ch. 9, the third-order step)
+__device__ __forceinline__ double sqrt(double x) {
+  const u64 b = bits_of(x);
+  const uint32_t ex = (hi32(b) >> 20) & 0x7ff;
+  const uint32_t odd = (ex & 1u) ^ 1u;                       // ex even: the unbiased exponent is odd
+  const u64 m = ((b << 11) | 0x8000000000000000ull) >> (1u - odd);   // units of 2^-64: [1/4, 1/2) or [1/2, 1)
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(__uint2float_rz(hi32(m)) * 0x1p-32f));   // in [1, 2]
+  const uint32_t y = min((uint32_t)(y0 * 0x1p31f), 0xffffff00u) - 0x400u;   // units of 2^-31, a little low
+  const u64 my = mul_wide(hi32(m), y) + __umulhi(lo32(m), y);        // m y, units of 2^-63, below 1
+  const u64 e = (1ull << 62) - (mul_wide(hi32(my), y) + __umulhi(lo32(my), y));   // 1 - m y^2, units of 2^-62, below 2^-19
+  const uint32_t eh = (uint32_t)(e >> 20);                   // units of 2^-42
+  const u64 g = (e >> 1) + ((mul_wide(eh, eh) * 3) >> 25);    // e/2 + 3 e^2/8, units of 2^-62
+  const u64 u = (my << 1) + (mul_hi(my, g) << 3);            // units of 2^-64: the root, in [1/2, 1)
+  const double r = double_of((u >> 11) + (((u64)((((ex + 1u) >> 1) + 510u) << 20) << 32) | ((lo32(u) >> 10) & 1u)));
+  if (hi32(b) - 0x00100000u >= 0x7fe00000u) return sqrt_any(x);   // zero, subnormal, negative, infinite, NaN
+  return r;
 }
 
 }  // namespace fm
