@@ -176,7 +176,8 @@ typedef struct wg_options {
   int32_t block_threads;   /* threads per block, a multiple of 32: up to 512 (FP64),   */
                            /* 256 (FP32), 128 (ensembles); 0 = one block per SM for    */
                            /* one FP64 member, 256 for one FP32 member, 64 for         */
-                           /* ensembles                                                */
+                           /* ensembles (joined to blocks of up to 1,024 in the        */
+                           /* wavefront where the states fill the GPU)                 */
   int32_t ring_days;       /* days of vertical outputs buffered between the vertical
                               balance run ahead and routing; 0 = as many as fit in 8 GB
                               or an eighth of the free device memory, the smaller */

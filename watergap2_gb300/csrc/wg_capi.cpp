@@ -144,7 +144,7 @@ void place_warps(const std::vector<int32_t> &seq, const uint32_t *cls, int n, co
 }
 
 wg_status build_topology(int n, const int32_t *down, const int32_t *rout_order, const uint32_t *cls,
-                         const WarpLayout *lay, Topology &t, const int32_t *node_of) {
+                         const WarpLayout *lay, Topology &t, const int32_t *node_of, bool heavy_first) {
   for (int i = 0; i < n; ++i)
     if (down[i] < -1 || down[i] >= n || down[i] == i) return WG_ERR_TOPOLOGY;
   std::vector<int32_t> order;
@@ -251,9 +251,12 @@ wg_status build_topology(int n, const int32_t *down, const int32_t *rout_order, 
   if (lay && lay->idle_warp >= 0) {
     place_warps(seq, cls, n, *lay, worder);
   } else {
+    // the classes evenly spread over the slots; heavy_first: the cells with the most water
+    // bodies first, for blocks whose warps take states in slot order until a step's are done
     std::map<uint32_t, int> seen;
     std::vector<std::pair<double, int>> key(wfull);
-    for (int w = 0; w < wfull; ++w) key[w] = {(seen[wcls[w]]++ + 0.5) / count[wcls[w]], w};
+    for (int w = 0; w < wfull; ++w)
+      key[w] = {heavy_first ? -(double)__builtin_popcount(wcls[w]) : (seen[wcls[w]]++ + 0.5) / count[wcls[w]], w};
     std::stable_sort(key.begin(), key.end());
     for (int k = 0; k < wfull; ++k) worder[k] = key[k].second;
     if (W > wfull) worder[W - 1] = W - 1;
@@ -380,9 +383,35 @@ void join_uploads(wg_ctx *ctx) {
 constexpr int kDataDays = 65;
 
 bool valid_block_threads(int threads, int precision, int members) {
-  const int mx = members > 1 ? PipeBounds<float, true>::threads
+  const int mx = members > 1 ? 128
                              : (precision == 0 ? Bounds<double>::threads : Bounds<float>::threads);
   return threads >= 32 && threads <= mx && threads % 32 == 0;
+}
+
+// An ensemble's states for every thread that the GPU holds of its wavefront.
+size_t states_per_thread(const wg_ctx *ctx) {
+  int nsm = 0;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+  return ctx->members > 1 && nsm > 0 ? ctx->nstate() / ((size_t)nsm * PipeBounds<float, true>::threads) : 0;
+}
+
+// An ensemble's launches for the context's block size. Wavefront: blocks are joined up to
+// the kernel's 512 threads where that still fills the GPU -- the more warps share a
+// block's states, the more evenly a step's work spreads over them; fewer states than
+// that are spread over as many SMs as there are blocks. Vertical balance ahead, whose
+// threads share nothing: on the second stream as many blocks as the GPU holds, by
+// itself one (cell, member) per thread, so that blocks start as SMs come free.
+void set_ensemble_shape(wg_ctx *ctx) {
+  constexpr int kMost = PipeBounds<float, true>::threads;
+  ctx->layout.join = 1;
+  while (ctx->threads * ctx->layout.join * 2 <= kMost) ctx->layout.join *= 2;
+  if (states_per_thread(ctx) < 1 ||
+      ctx->blocks_fused / ctx->layout.join < pipeline_max_blocks<float>(true, true, ctx->threads * ctx->layout.join))
+    ctx->layout.join = 1;
+  ctx->threads_va = std::min(ctx->threads, 64);
+  const size_t need = std::min<size_t>((ctx->nstate() + ctx->threads_va - 1) / ctx->threads_va, (size_t)1 << 30);
+  ctx->blocks_va_alone = (int)need;
+  ctx->blocks_va = std::min(vertical_ahead_max_blocks<float>(true, ctx->threads_va), (int)need);
 }
 
 // Single-member contexts: one block per SM with an equal share of the cells in
@@ -1155,7 +1184,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
       if (ctx->glwd.unit_of[i] >= 0) node_of[i] = first[ctx->glwd.unit_of[i]];
   }
   wg_status st = build_topology(n, r->downstream, r->rout_order, cls.data(), &ctx->layout, ctx->topo,
-                                aggr ? node_of.data() : nullptr);
+                                aggr ? node_of.data() : nullptr, states_per_thread(ctx.get()) >= 1);
   if (st != WG_OK) {
     if (aggr && st == WG_ERR_TOPOLOGY)
       t_create_err = "GLWD units: the cells of a unit drain out of it and back in (no wavefront order)";
@@ -1467,7 +1496,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     if (cudaStreamCreateWithFlags(&ctx->va_stream, cudaStreamNonBlocking) != cudaSuccess) return WG_ERR_CUDA;
     for (cudaEvent_t *e : {&ctx->ev_fork, &ctx->ev_va, &ctx->ev_pipe[0], &ctx->ev_pipe[1]})
       if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return WG_ERR_CUDA;
-    ctx->blocks_va = std::min(vertical_ahead_max_blocks<float>(true, th), need);
+    set_ensemble_shape(ctx.get());
   }
   if (ctx->layout.idle_warp >= 0) {
     st = setup_step_flags(ctx.get());
@@ -1909,7 +1938,7 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
       const cudaError_t pe = launch_pet(c, ctx->forcing, ring, doy0, fday0, ndays, a, b, ctx->va_stream);
       if (pe != cudaSuccess) return pe;
       return launch_vertical_ahead(c, s, ctx->forcing, ctx->mem, ctx->balance, ring, doy0, fday0, ndays, a, b,
-                                   ctx->blocks_va, ctx->threads, ctx->va_stream, ctx->mon, oday0);
+                                   ctx->blocks_va, ctx->threads_va, ctx->va_stream, ctx->mon, oday0);
     };
     cudaError_t e = cudaEventRecord(ctx->ev_fork, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->va_stream, ctx->ev_fork, 0);
@@ -1953,7 +1982,9 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
     }
     if (!ov || a == t_b) {
       e = launch_vertical_ahead(c, s, ctx->forcing, ctx->mem, ctx->balance, ring, doy0, fday0, ndays, a, b,
-                                ctx->blocks_fused, ctx->threads, ctx->stream, ctx->mon, oday0);
+                                ctx->members > 1 ? ctx->blocks_va_alone : ctx->blocks_fused,
+                                ctx->members > 1 ? ctx->threads_va : ctx->threads, ctx->stream, ctx->mon, oday0,
+                                states_per_thread(ctx) >= 8);
       ctx->launches++;
     }
     if (ev) cudaEventRecord(ev[1], ctx->stream);
@@ -2624,7 +2655,7 @@ wg_status wg_launch_shape(wg_ctx *ctx, int32_t threads, int32_t blocks) {
   ctx->threads = threads;
   ctx->blocks_fused = std::min(blocks > 0 ? std::min(blocks, maxb) : maxb, need);
   ctx->blocks_route = std::min(blocks > 0 ? std::min(blocks, maxr) : maxr, need);
-  if (ens && ctx->precision == 1) ctx->blocks_va = std::min(vertical_ahead_max_blocks<float>(true, threads), need);
+  if (ens && ctx->precision == 1) set_ensemble_shape(ctx);
   return WG_OK;
 }
 

@@ -142,7 +142,8 @@ struct wg_ctx {
   bool ens_overlap = false;
   cudaStream_t va_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_va = nullptr, ev_pipe[2] = {nullptr, nullptr};
-  int blocks_va = 0;                       // grid of the vertical-ahead launches on va_stream
+  int blocks_va = 0, threads_va = 0;       // an ensemble's vertical-ahead launches on va_stream,
+  int blocks_va_alone = 0;                 // ... and on the context's stream
   bool timing = false;                     // CUDA events around each launch pair of wg_run_steps
   std::vector<cudaEvent_t> tev;            // 3 per recorded launch pair
   size_t tev_used = 0;

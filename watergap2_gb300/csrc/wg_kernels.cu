@@ -409,8 +409,11 @@ __device__ __forceinline__ void va_cell(const DevCellsT<R> &c, const DevStateT<R
 // ring buffer.  Results equal the in-wavefront computation: the vertical balance of
 // such a cell reads nothing routing writes.
 // OUT: the vertical balance's monthly output grids too (DevMonthly::vert, FP64 single member).
-template <class R, bool ENS, bool OUT = false>
-__global__ void __launch_bounds__(VaBounds<R, ENS>::threads, VaBounds<R, ENS>::min_blocks) k_vertical_ahead(DevCellsT<R> c, DevStateT<R> st, DevForcing f,
+// BLOCKS: of 256 threads an SM holds; an ensemble of many states per thread the GPU holds
+// gains more from the third (80 registers instead of 110, 92 bytes of spills) than it
+// loses: 67k cells x 64 members, 90 days 8.7 -> 7.7 ms, 67k x 12 the same, 67k x 2, 40 days 0.71 -> 0.78.
+template <class R, bool ENS, bool OUT = false, int BLOCKS = VaBounds<R, ENS>::min_blocks>
+__global__ void __launch_bounds__(VaBounds<R, ENS>::threads, BLOCKS) k_vertical_ahead(DevCellsT<R> c, DevStateT<R> st, DevForcing f,
                                                         DevMembers mem, DevBalance b, DevRingT<R> ring, int doy0,
                                                         int fday0, int ndays, int t_b, int t_e, DevMonthly mon,
                                                         int oday0) {
@@ -474,6 +477,40 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
     one_ue = c.up_ptr[gtid + 1];
     if (one_ue > one_u) one_up = c.up_idx[one_u];
   }
+  // Ensembles that fill the GPU (blocks of more than 128 threads): the warps of a block
+  // take its states 32 at a time from a shared counter, in slot order, which puts the
+  // cells with the most water bodies first. Dealt out to the warps in advance a third of
+  // the time went by in waiting at the steps' barriers for the one whose states took
+  // longest (67k cells x 64 members, 90 days: 20.5 -> 16.5 ms; 9k x 33, 40 days: 1.72 ->
+  // 1.49). 64 states go to each block in turn: 128 or 512 in a row spread the active part
+  // of a class unevenly (with blocks of 512 and no class first 18.9 as 64, 21.6 ms), 32
+  // halve the use of a fetched sector (19.3).
+  // A block's states stay its own, so that what one of its warps wrote in a step the
+  // others read after the barrier. The counter only grows: each warp of the block takes
+  // one number past a step's. Smaller ensembles, about a state a thread, have nothing to
+  // share out and keep the plain mapping.
+  const bool take = ENS && blockDim.x > 128;
+  [[maybe_unused]] __shared__ unsigned s_taken;
+  [[maybe_unused]] unsigned step_base = 0, block_items = 0;
+  if (take) {
+    const size_t groups = (N + 63) / 64;
+    block_items = 2 * (unsigned)(groups / gridDim.x + (blockIdx.x < groups % gridDim.x ? 1 : 0));
+    if (threadIdx.x == 0) s_taken = 0;
+    __syncthreads();
+  }
+  // this lane's next state of the step after state i (-1: its first), -1 when there is none;
+  // N and more: none for this lane, but the warp has one
+  auto next_state = [&](long long i) -> long long {
+    if (!take) {
+      i = i < 0 ? gtid : i + gstride;
+      return i < (long long)N ? i : -1;
+    }
+    unsigned k = 0;
+    if ((threadIdx.x & 31) == 0) k = atomicAdd(&s_taken, 1u) - step_base;
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (k >= block_items) return -1;
+    return ((((long long)(k >> 1) * gridDim.x + blockIdx.x) * 2 + (k & 1)) << 5) + (threadIdx.x & 31);
+  };
   int row_t = t_b % sync.rows;   // t % sync.rows
   for (int t = va_only ? t_e : t_b; t < t_e; ++t, row_t = row_t + 1 == sync.rows ? 0 : row_t + 1) {
     if (flow && t > t_b) {
@@ -548,8 +585,9 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
       }
       // state index i always belongs to thread i mod gstride, so a cell's state is read
       // and written by one thread; only upstream outflows cross threads (read via L2)
-      for (long long i = gtid; i < (long long)N; i += gstride) {
-        const int s0 = ENS ? (int)(i / M) : (int)i;
+      for (long long i = ENS ? next_state(-1) : gtid; ENS ? i >= 0 : i < (long long)N; i = ENS ? next_state(i) : i + gstride) {
+        if (ENS && i >= (long long)N) continue;
+        const int s0 = !ENS ? (int)i : N >> 32 ? (int)(i / M) : (int)((unsigned)i / (unsigned)M);
         const int mm = ENS ? (int)(i - (long long)s0 * M) : 0;
         const int dbase = kd * (t - (one ? one_off : c.offset[s0]));
         if (dbase < 0 || dbase >= ndays) continue;   // this cell's wavefront has not reached it yet / is done
@@ -824,6 +862,7 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
          }   // cells of the unit
         }   // days of the step
       }
+      if (take) step_base += block_items + blockDim.x / 32;
     }
     if (flow) {
       // publish step t: every lane's writes of this step (fence, one instruction for
@@ -1058,7 +1097,14 @@ template <class R>
 cudaError_t launch_vertical_ahead(const DevCellsT<R> &c, const DevStateT<R> &s, const DevForcing &f,
                                   const DevMembers &mem, const DevBalance &b, const DevRingT<R> &ring, int doy0,
                                   int fday0, int ndays, int t_b, int t_e, int blocks, int threads, cudaStream_t st,
-                                  const DevMonthly &mon, int oday0) {
+                                  const DevMonthly &mon, int oday0, bool dense) {
+  if constexpr (std::is_same<R, float>::value) {
+    if (mem.members > 1 && dense) {
+      k_vertical_ahead<R, true, false, VaBounds<R, true>::min_blocks + 1><<<blocks, threads, 0, st>>>(
+          c, s, f, mem, b, ring, doy0, fday0, ndays, t_b, t_e, mon, oday0);
+      return cudaGetLastError();
+    }
+  }
   if (mem.members > 1)
     k_vertical_ahead<R, true><<<blocks, threads, 0, st>>>(c, s, f, mem, b, ring, doy0, fday0, ndays, t_b, t_e, mon,
                                                           oday0);
@@ -1169,6 +1215,10 @@ cudaError_t launch_pipeline(bool fused, const DevCellsT<R> &c, const DevStateT<R
   if (vaw && (idle_warp < 0 || mem.members > 1 || vw.warps != lay.va_warps)) return cudaErrorInvalidConfiguration;
   DevVaWork vwk = vw;
   if (!vaw) vwk.warps = vwk.nitems = 0;
+  if (mem.members > 1 && lay.join > 1 && blocks % lay.join == 0) {
+    blocks /= lay.join;
+    threads *= lay.join;
+  }
   void *args[] = {(void *)&c,    (void *)&s,    (void *)&v,     (void *)&f,     (void *)&mem,   (void *)&b,
                   (void *)&ring, (void *)&sync, (void *)&outq,  (void *)&qst,   (void *)&doy0,  (void *)&fday0,
                   (void *)&oday0, (void *)&ndays, (void *)&t_b, (void *)&t_e, (void *)&cell_warps,
@@ -1228,7 +1278,7 @@ cudaError_t launch_balance_sum(const DevCellsT<R> &c, const DevStateT<R> &s, int
   template cudaError_t launch_vertical_ahead<R>(const DevCellsT<R> &, const DevStateT<R> &, const DevForcing &,   \
                                                 const DevMembers &, const DevBalance &, const DevRingT<R> &, int,  \
                                                 int, int, int, int, int, int, cudaStream_t, const DevMonthly &,   \
-                                                int);                                                              \
+                                                int, bool);                                                              \
   template cudaError_t launch_volume<R>(const DevCellsT<R> &, const DevStateT<R> &, int, double *, cudaStream_t); \
   template cudaError_t launch_balance_sum<R>(const DevCellsT<R> &, const DevStateT<R> &, int, const DevBalance &,  \
                                              const double *, double *, int *, cudaStream_t);

@@ -19,10 +19,11 @@ template <> struct Bounds<float> { static constexpr int threads = 256, min_block
 // registers: two blocks per SM, no spills
 template <class R, bool ENS> struct VaBounds : Bounds<R> {};
 template <> struct VaBounds<float, true> { static constexpr int threads = 256, min_blocks = 2; };
-// the ensemble's wavefront kernel is bound by load latency: at most 128 threads
-// per block and 64 registers, so that an SM holds 32 warps of it (no spills)
+// the ensemble's wavefront kernel is bound by load latency: 64 registers, so that an
+// SM holds 32 warps of it, in one block where there are states for all (the warps of a
+// block share its states out among themselves: two blocks of 512 17.1 ms, one 16.5)
 template <class R, bool ENS> struct PipeBounds : Bounds<R> {};
-template <> struct PipeBounds<float, true> { static constexpr int threads = 128, min_blocks = 8; };
+template <> struct PipeBounds<float, true> { static constexpr int threads = 1024, min_blocks = 1; };
 // the single-member FP64 wavefront with vertical-balance warps in the same block: 16
 // warps, four per SM sub-partition, so that a thread has 128 registers
 template <class R, bool ENS, bool VAW> struct WaveBounds : PipeBounds<R, ENS> {};
@@ -38,6 +39,7 @@ struct WarpLayout {
   bool va_on = false;  // the wavefront launches carry the next chunk's vertical balance
   int blocks = 0;
   int threads = 0;
+  int join = 1;        // ensembles: blocks of the launch shape that a wavefront block joins
 };
 cudaError_t upload_fastmath_tables(const unsigned long long exp2_tab[256], const ulonglong2 log2_tab[256]);
 cudaError_t launch_math_eval(int fn, const double *x, const double *y, double *out, size_t n, cudaStream_t st);
@@ -79,7 +81,7 @@ template <class R>
 cudaError_t launch_vertical_ahead(const DevCellsT<R> &c, const DevStateT<R> &s, const DevForcing &f,
                                   const DevMembers &mem, const DevBalance &b, const DevRingT<R> &ring, int doy0,
                                   int fday0, int ndays, int t_b, int t_e, int blocks, int threads, cudaStream_t st,
-                                  const DevMonthly &mon, int oday0);
+                                  const DevMonthly &mon, int oday0, bool dense = false);
 template <class R>
 cudaError_t launch_volume(const DevCellsT<R> &c, const DevStateT<R> &s, int M, double *vol, cudaStream_t st);
 template <class R>

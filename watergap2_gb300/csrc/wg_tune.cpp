@@ -198,7 +198,7 @@ wg_status wg_autotune(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t ndays, i
   if (t_begin < 0 || t_begin + trial_steps > total) return WG_ERR_INVALID;
   cudaSetDevice(ctx->device);
   const int th0 = ctx->threads, ch0 = ctx->chunk_steps;
-  const int bf0 = ctx->blocks_fused, br0 = ctx->blocks_route, bv0 = ctx->blocks_va;
+  const int bf0 = ctx->blocks_fused, br0 = ctx->blocks_route, bv0 = ctx->blocks_va, tv0 = ctx->threads_va, ba0 = ctx->blocks_va_alone;
   const bool eo0 = ctx->ens_overlap;
   const WarpLayout lay0 = ctx->layout;
   int32_t tmp = 0;
@@ -224,6 +224,8 @@ wg_status wg_autotune(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t ndays, i
     ctx->blocks_fused = bf0;
     ctx->blocks_route = br0;
     ctx->blocks_va = bv0;
+    ctx->threads_va = tv0;
+    ctx->blocks_va_alone = ba0;
     ctx->layout = lay0;
   };
   // ensembles: without and with the stream overlap, the wavefront launch on all
