@@ -1005,7 +1005,7 @@ static void glwd_aggregate(const wg_ctx::Glwd &g, const double *nus, double *out
 
 // Water temperature buffers: state at the reference's start values (15 degC, no
 // ice: routing.cpp:172-197), the per-cell inputs in slot order.
-static wg_status setup_water_temp(wg_ctx *ctx, const wg_region *r) {
+static wg_status setup_water_temp(wg_ctx *ctx, const wg_region *r, const std::vector<double> &bw) {
   const int n = ctx->n;
   const size_t N = ctx->nstate();
   DevWaterTemp &w = ctx->wt;
@@ -1024,9 +1024,24 @@ static wg_status setup_water_temp(wg_ctx *ctx, const wg_region *r) {
   w.len_check = upload_slots<double>(ctx, len, st);
   w.lake_km2 = upload_slots<double>(ctx, lake, st);
   w.res_km2 = upload_slots<double>(ctx, res, st);
-  w.ll_pct = upload_slots<double>(ctx, ll, st);
-  w.lw_pct = upload_slots<double>(ctx, lw, st);
-  w.gw_pct = upload_slots<double>(ctx, gw, st);
+  for (std::vector<double> *v : {&ll, &lw, &gw})
+    for (double &x : *v) x /= 100.;
+  w.ll_part = upload_slots<double>(ctx, ll, st);
+  w.lw_part = upload_slots<double>(ctx, lw, st);
+  w.gw_part = upload_slots<double>(ctx, gw, st);
+  // the volumes above the thermocline (calcWaterTemp.cpp:1313-1324) and the river bed's
+  // terms of the flow depth (calcWaterTemp.cpp:1110-1116)
+  std::vector<double> bed(n), bed2(n);
+  for (int i = 0; i < n; ++i) {
+    lake[i] = lake[i] * (9.52 * std::pow(std::sqrt(2 * lake[i]), 0.425));
+    res[i] = res[i] * (9.52 * std::pow(std::sqrt(3 * res[i] / std::sqrt(3.)), 0.425));
+    bed[i] = bw[i] / (4. * 1000.);
+    bed2[i] = bw[i] / 1000. * bw[i] / (16. * 1000.);
+  }
+  w.lake_therm = upload_slots<double>(ctx, lake, st);
+  w.res_therm = upload_slots<double>(ctx, res, st);
+  w.bed = upload_slots<double>(ctx, bed, st);
+  w.bed2 = upload_slots<double>(ctx, bed2, st);
   if (st != WG_OK) return st;
   std::vector<double> t15(6 * N, 15.), zero(6 * N, 0.);
   cudaError_t e = cudaMemcpy(w.temp, t15.data(), 6 * N * sizeof(double), cudaMemcpyHostToDevice);
@@ -1468,7 +1483,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
   st = ctx->precision == 0 ? broadcast_state(ctx.get(), ctx->sd, &init) : broadcast_state(ctx.get(), ctx->sf, &init);
   if (st != WG_OK) return st;
   if (opt->water_temp) {
-    st = setup_water_temp(ctx.get(), r);
+    st = setup_water_temp(ctx.get(), r, h.bw);
     if (st != WG_OK) return st;
   }
   if (opt->water_use) {

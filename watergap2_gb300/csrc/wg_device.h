@@ -240,7 +240,9 @@ struct DevWaterTemp {
   const float *gwt;          // [n] yearly groundwater temperature [degC]
   const double *len_check;   // [n] river length as read (55: no river in the cell)
   const double *lake_km2, *res_km2;   // [n] global lake and reservoir area [km2]
-  const double *ll_pct, *lw_pct, *gw_pct;   // [n] local lake, local and global wetland [% of the cell]
+  const double *lake_therm, *res_therm; // [n] their volumes above the thermocline [km3]
+  const double *ll_part, *lw_part, *gw_part;   // [n] local lake, local and global wetland [part of the cell]
+  const double *bed, *bed2;  // [n] river bed: bottom width / 4 [km], its square
   double *qst_t;             // [max_days][nstation] river temperature at the stations
   int32_t enabled;
 };

@@ -251,7 +251,7 @@ __device__ __forceinline__ double rcp_pos(double x) {
 
 __device__ __noinline__ double div_any(double a, double b) { return a / b; }
 
-// a / b to half an ulp and 2^-8 more for normal a and b with a normal quotient (a = 0
+// a / b to 0.52 ulp for normal a and b with a normal quotient (a = 0
 // gives 0 with the quotient's sign), anything else through the general division
 __device__ __forceinline__ double div(double a, double b) {
   const u64 ab = bits_of(a), bb = bits_of(b);
@@ -269,7 +269,8 @@ __device__ __forceinline__ double div(double a, double b) {
 
 __device__ __noinline__ double sqrt_any(double x) { return ::sqrt(x); }
 
-// square root of a positive normal number to half an ulp and 2^-8 more: m in [1/4, 1),
+// square root of a positive normal number to half an ulp and 2^-5 more (the fourth term
+// of the series and the truncated products):  m in [1/4, 1),
 // the single-precision reciprocal root y of its leading bits, e = 1 - m y^2, then
 // m y (1 + e/2 + 3 e^2/8) (Markstein 2000, ch. 9, the third-order step)
 __device__ __forceinline__ double sqrt(double x) {

@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
             if constexpr (WT) tq = ld_relaxed(t_prev0 + ui);
             if (!is_outflow(sync, q) || (WT && !is_outflow(sync, tq))) break;
             pre_up += q;
-            if constexpr (WT) pre_e += q * WT_RC * (tq + WT_CONV_K);
+            if constexpr (WT) pre_e += q * (tq + WT_CONV_K);
             ++k;
           }
           if (__all_sync(0xffffffffu, k >= k_e)) break;
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
                                     : ENS ? __ldcg(q_prev + ui) : upstream_value<!FUSED>(sync, q_prev + ui, failed);
               up += qu;
               if constexpr (WT)   // the energy the inflow carries (calcWaterTemp.cpp:76-83)
-                e_up += qu * WT_RC * (upstream_value<!FUSED>(sync, t_prev0 + (size_t)kk * N + ui, failed) + WT_CONV_K);
+                e_up += qu * (upstream_value<!FUSED>(sync, t_prev0 + (size_t)kk * N + ui, failed) + WT_CONV_K);
             }
             return up;
           };
@@ -734,8 +734,8 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
           else st_outflow(q_now + si, (double)tv);
           if constexpr (WT) {
             // a cell without continental area keeps the reference's initial 15 degrees (routing.cpp:174)
-            const double tr = nocont ? 15. : wtd.river((double)rs.river, (double)c.bw[s], (double)c.rlen[s],
-                                                       (double)c.cfa[s], (double)o.owpet);
+            const double tr = nocont ? 15. : wtd.river((double)rs.river, (double)c.rlen[s], (double)c.cfa[s],
+                                                       (double)o.owpet);
             st_outflow(t_now0 + (size_t)kk * N + si, tr);
             const int stw = c.station[s];
             if (stw >= 0) wtp.qst_t[(size_t)(oday0 + d) * c.nstation + stw] = tr;
