@@ -1,10 +1,7 @@
 """The fixed-point quotient and square root of the water temperature, compiled from
 their header: random and edge mantissas over the exponents, and everything that is
-not a normal number as the hardware has it.
-
-Bounds in ulp: half an ulp of the final rounding plus, for the quotient, that of the
-reciprocal (0.01) and of one truncated product; for the root, four truncated products
-(2^-8 each at most) and the series' fourth term (2^-7.5)."""
+not a normal number as the hardware has it. Both round correctly, so the
+results are the bits of the host's."""
 import ctypes
 import os
 import subprocess
@@ -13,7 +10,6 @@ import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
-LD = np.longdouble
 
 SRC = r"""
 #include <cuda_runtime.h>
@@ -55,19 +51,14 @@ def run(tmp_path_factory):
     return call
 
 
-def _ulp(got, ref):
-    return np.abs(LD(got) - ref) / np.spacing(np.abs(ref).astype(np.float64)).astype(LD)
-
-
-@pytest.mark.skipif(np.finfo(LD).nmant < 63, reason="no wider type to compare with")
 def test_rounding(run):
     rng = np.random.default_rng(3)
     m = np.concatenate([1 + rng.random(100000), 1 + np.ldexp(1.0, -np.arange(1, 53)), 2 - np.ldexp(1.0, -np.arange(1, 53))])
     a = np.ldexp(m, rng.integers(-300, 300, m.size)) * rng.choice([-1, 1], m.size)
     b = np.ldexp(rng.permutation(m), rng.integers(-300, 300, m.size))
-    assert _ulp(run(0, a, b), LD(a) / LD(b)).max() < 0.52
+    assert np.array_equal(run(0, a, b), a / b)
     x = np.concatenate([np.abs(a), np.nextafter(np.ldexp(1.0, np.arange(-1000, 1000)), 0), np.ldexp(1.0, np.arange(-1000, 1000))])
-    assert _ulp(run(1, x, x), np.sqrt(LD(x))).max() < 0.5 + 2.0 ** -5
+    assert np.array_equal(run(1, x, x), np.sqrt(x))
 
 
 def test_not_normal(run):
@@ -76,9 +67,5 @@ def test_not_normal(run):
     with np.errstate(all="ignore"):
         want, root = a / b, np.sqrt(v)
     got = run(0, a, b)
-    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.signbit(got[want == 0]), np.signbit(want[want == 0]))
-    ok = np.isfinite(want) & (want != 0)
-    assert np.array_equal(got[~ok], want[~ok], equal_nan=True)
-    assert np.all(np.abs(got[ok] - want[ok]) <= np.spacing(np.abs(want[ok])))
-    assert np.array_equal(run(1, v, v)[[0, 1, 4, 5, 6]], root[[0, 1, 4, 5, 6]], equal_nan=True)
-    assert np.isnan(run(1, v, v)[3]) and np.all(np.abs(run(1, v, v)[7:8] - root[7:8]) <= np.spacing(root[7:8]))
+    assert np.array_equal(got, want, equal_nan=True) and np.array_equal(np.signbit(got[want == 0]), np.signbit(want[want == 0]))
+    assert np.array_equal(run(1, v, v), root, equal_nan=True)

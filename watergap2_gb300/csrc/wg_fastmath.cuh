@@ -251,17 +251,21 @@ __device__ __forceinline__ double rcp_pos(double x) {
 
 __device__ __noinline__ double div_any(double a, double b) { return a / b; }
 
-// a / b to 0.52 ulp for normal a and b with a normal quotient (a = 0
-// gives 0 with the quotient's sign), anything else through the general division
+// a / b, correctly rounded (the midpoint next to the approximate quotient, times b,
+// compared with a): normal a and b with a normal quotient, and a = 0; anything else
+// through the general division. 130 cycles per warp (the
+// root 127), 108 without the last comparison
 __device__ __forceinline__ double div(double a, double b) {
   const u64 ab = bits_of(a), bb = bits_of(b);
   const int ea = (int)((hi32(ab) >> 20) & 0x7ff), eb = (int)((hi32(bb) >> 20) & 0x7ff);
   const u64 sign = (ab ^ bb) & 0x8000000000000000ull;
-  u64 q = mul_hi((ab << 11) | 0x8000000000000000ull, rcp_mant((bb << 11) | 0x8000000000000000ull));
+  const u64 am = (ab << 11) | 0x8000000000000000ull, bm = (bb << 11) | 0x8000000000000000ull;
+  u64 q = mul_hi(am, rcp_mant(bm));
   const uint32_t low = (hi32(q) >> 31) ^ 1u;                 // the quotient of the mantissas is below 1
   q <<= low;
   const int e = ea - eb + 1022 - (int)low;                   // biased exponent less one
-  const double r = double_of(((q >> 11) + (((u64)((uint32_t)e << 20) << 32) | ((lo32(q) >> 10) & 1u))) | sign);
+  const uint32_t up = __umul64hi((q & ~0x7ffull) | 0x400u, bm) < am >> (low ^ 1u);
+  const double r = double_of(((q >> 11) + (((u64)((uint32_t)e << 20) << 32) | up)) | sign);
   if ((unsigned)(eb - 1) >= 2046u || ((unsigned)(ea - 1) >= 2046u && (ab << 1) != 0) || (ea && (unsigned)(e - 1) >= 2043u))
     return div_any(a, b);
   return ea ? r : double_of(sign);
@@ -269,10 +273,10 @@ __device__ __forceinline__ double div(double a, double b) {
 
 __device__ __noinline__ double sqrt_any(double x) { return ::sqrt(x); }
 
-// square root of a positive normal number to half an ulp and 2^-5 more (the fourth term
-// of the series and the truncated products):  m in [1/4, 1),
+// square root of a positive normal number, correctly rounded: m in [1/4, 1),
 // the single-precision reciprocal root y of its leading bits, e = 1 - m y^2, then
-// m y (1 + e/2 + 3 e^2/8) (Markstein 2000, ch. 9, the third-order step)
+// m y (1 + e/2 + 3 e^2/8) (Markstein 2000, ch. 9, the third-order step), and the square
+// of the midpoint next to it compared with m
 __device__ __forceinline__ double sqrt(double x) {
   const u64 b = bits_of(x);
   const uint32_t ex = (hi32(b) >> 20) & 0x7ff;
@@ -286,7 +290,9 @@ __device__ __forceinline__ double sqrt(double x) {
   const uint32_t eh = (uint32_t)(e >> 20);                   // units of 2^-42
   const u64 g = (e >> 1) + ((mul_wide(eh, eh) * 3) >> 25);    // e/2 + 3 e^2/8, units of 2^-62
   const u64 u = (my << 1) + (mul_hi(my, g) << 3);            // units of 2^-64: the root, in [1/2, 1)
-  const double r = double_of((u >> 11) + (((u64)((((ex + 1u) >> 1) + 510u) << 20) << 32) | ((lo32(u) >> 10) & 1u)));
+  const u64 mid = (u & ~0x7ffull) | 0x400u;
+  const uint32_t up = __umul64hi(mid, mid) < m;
+  const double r = double_of((u >> 11) + (((u64)((((ex + 1u) >> 1) + 510u) << 20) << 32) | up));
   if (hi32(b) - 0x00100000u >= 0x7fe00000u) return sqrt_any(x);   // zero, subnormal, negative, infinite, NaN
   return r;
 }

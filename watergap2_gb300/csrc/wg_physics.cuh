@@ -43,6 +43,7 @@ template <> struct M<double> {
   static __device__ __forceinline__ double exp_neg(double x) { return fm::exp_neg(x); }   // exp(-x), x >= 0
   static __device__ __forceinline__ double pow(double x, double y) { return fm::pow(x, y); }
   static __device__ __forceinline__ double rcp(double x) { return fm::rcp_pos(x); }   // x normal, nonzero
+  static __device__ __forceinline__ double sqrt_(double x) { return fm::sqrt(x); }
   static __device__ __forceinline__ double fabs_(double x) { return fabs(x); }
   // 1 - exp(-k) as the reference writes it (its rounding is the parity target)
   static __device__ __forceinline__ double one_m_exp_neg(double k, double e) { return 1. - e; }
@@ -52,6 +53,7 @@ template <> struct M<float> {
   static __device__ __forceinline__ float exp_neg(float x) { return expf(-x); }
   static __device__ __forceinline__ float pow(float x, float y) { return (x > 0.f) ? powf(x, y) : 0.f; }
   static __device__ __forceinline__ float rcp(float x) { return 1.0f / x; }
+  static __device__ __forceinline__ float sqrt_(float x) { return sqrtf(x); }
   static __device__ __forceinline__ float fabs_(float x) { return fabsf(x); }
   // 1 - exp(-k) without the cancellation of the subtraction: a slow river's
   // small k leaves 1 - expf(-k) with a relative error of 1e-7 / k in FP32
@@ -756,7 +758,7 @@ __device__ __forceinline__ R river_velocity(const DevCellsT<R> &c, int s, R rive
     csa = depth * (R(2.0) * depth + bw);
   } else {
     csa = (S * c.inv_len[s]) * R(1000000.);
-    depth = -bw * R(0.25) + sqrt(bw * bw * R(1.0 / 16.0) + R(0.5) * csa);
+    depth = -bw * R(0.25) + m::sqrt_(bw * bw * R(1.0 / 16.0) + R(0.5) * csa);
   }
   const R wp = bw + R(2.0 * 2.23606797749979) * depth;   // 2 sqrt(5)
   const R hr = csa * m::rcp(wp);
