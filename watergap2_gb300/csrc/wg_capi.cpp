@@ -327,7 +327,7 @@ struct HostConsts {
   // one vector per DevCellsT field of type R
 #define WG_RFIELDS(X)                                                                                            \
   X(cfa) X(inv_cfa) X(mprec) X(alpha) X(pet_mxdy) X(mnetrad) X(mcwh) X(t_snowfz) X(t_snowmt) X(pcritgwa) X(gamma) \
-  X(albedo) X(albedo_snow) X(ddf_m) X(lai_min) X(lai_max) X(lai_s30) X(smax) X(inv_smax) X(fg) X(rgmax) X(built_up)         \
+  X(albedo) X(albedo_snow) X(ddf_m) X(lai_min) X(lai_max) X(lai_span) X(smax) X(inv_smax) X(fg) X(rgmax) X(built_up)         \
   X(t_gradnt) X(elev0) X(contfreq) X(area) X(area_f) X(gw_e) X(gw_ik) X(gw_ome) X(sw_k) X(sw_e) X(sw_ik)        \
   X(sw_ome) X(evx)                                                                                               \
   X(a6) X(ll100) X(maxs_ll) X(inv_maxs_ll) X(lw100) X(maxs_lw) X(inv_maxs_lw) X(la6) X(maxs_gl) X(inv_maxs_gl)  \
@@ -514,7 +514,7 @@ wg_status setup_step_flags(wg_ctx *ctx) {
   if (st != WG_OK) return st;
   if (!ctx->sync.wstep) return WG_ERR_NOMEM;
   ctx->sync.nwarps = W;
-  ctx->sync.flow = 0;   // measured on GB300: the grid barrier is 3.6 % faster (flags: wg_set_step_sync)
+  ctx->sync.flow = 0;   // slower than the waits for outflows and than the grid barrier (wg_set_step_sync)
   return WG_OK;
 }
 
@@ -1252,7 +1252,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     const float lmin = r->lct_lai_a[lct - 1] + r->lct_lai_b[lct - 1] * r->lai_max[i];   // lai.cpp:154 (float)
     h.lai_min[i] = lmin;
     h.lai_max[i] = r->lai_max[i];
-    h.lai_s30[i] = ((double)r->lai_max[i] - (double)lmin) / 30.0;
+    h.lai_span[i] = (double)r->lai_max[i] - (double)lmin;
     {   // the output grids' constants: Kc (lai.cpp:295-306, LAImin in float as there),
         // the first year's freshwater share (routing.cpp:1213), the global-lake and
         // reservoir shares, G_loc_lake / 100

@@ -56,7 +56,7 @@ struct DevCellsT {
   const int32_t *station;       // station index or -1
   // vertical balance
   const R *cfa, *inv_cfa, *mprec, *alpha, *pet_mxdy, *mnetrad, *mcwh, *t_snowfz, *t_snowmt, *pcritgwa, *gamma;
-  const R *albedo, *albedo_snow, *ddf_m, *lai_min, *lai_max, *lai_s30, *smax, *inv_smax, *fg, *rgmax, *built_up;
+  const R *albedo, *albedo_snow, *ddf_m, *lai_min, *lai_max, *lai_span, *smax, *inv_smax, *fg, *rgmax, *built_up;
   const R *t_gradnt, *elev0;
   const R *contfreq;            // continental share of the cell [%] (the monthly output grids)
   const R *band_dt;             // [nband][n] (elev_b - elev_0) * P_T_GRADNT

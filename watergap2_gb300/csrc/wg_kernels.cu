@@ -8,28 +8,35 @@
 //                  day d at step d + offset(n), offset = longest flow path -
 //                  distance of n to its outlet.  Every upstream cell of n then
 //                  has offset(n) - 1 and delivers day d's outflow exactly one step
-//                  earlier through a two-slot buffer, so one grid barrier per step
-//                  (or, optionally, per-warp step flags) is the only
-//                  synchronisation and every step keeps all cells busy.  Cells
+//                  earlier.  A cell waits for these outflows themselves (one FP64
+//                  member; rows of the outflow buffer per step), or all cells for
+//                  a grid barrier per step (ensembles, GLWD units, runs with
+//                  skipped cells) or, optionally, for per-warp step flags.  Cells
 //                  without a water body take their vertical balance from the ring
 //                  that k_vertical_ahead filled; the monthly output aggregates are
 //                  accumulated in its epilogue.  With ENS the cells carry
 //                  `members` independent states (ensemble members), innermost in
-//                  memory.  With VAW (one FP64 member) each block has five more
-//                  warps that run k_vertical_ahead's work for the next chunk
-//                  while the routing warps wait; with WT every cell also gets
+//                  memory.  With VAW (one FP64 member) each block's idle warp, any
+//                  further warps it has room for and the routing warps that are
+//                  done run k_vertical_ahead's work for the next chunk; with WT
+//                  every cell also gets
 //                  its water temperature (calcWTemp), the river temperature
 //                  travelling downstream beside the outflow.
+//  k_pet           potential evapotranspiration of a run's days, side by side,
+//                  into the ring.
 //  k_vertical_ahead  the vertical balance of the cells without a water body for
 //                  a chunk of days, state in registers, into the ring.
+//  k_state_rows / k_rows   state, output grids, water use and water temperature
+//                  into cell order for reading.
 //  k_math_eval     the FP64 path's exp/log/pow/reciprocal on arrays (tests).
 //  k_unf_forcing / k_gather_forcing  forcing uploads into the slot layout.
 //  k_volume / k_balance_sum   compensated (Neumaier) FP64 water-balance sums.
 //
 // Precision: R = double is the plain FP64 path; R = float keeps state and
 // fluxes in FP32 while confluence sums, the outflow buffer and all balance
-// sums stay FP64.  The grid barrier spins with an iteration limit: on timeout
-// it raises the context's error word and every block returns (no trap).
+// sums stay FP64.  The grid barrier and the waits for outflows spin with an
+// iteration limit: on timeout they raise the context's error word and every block
+// returns (no trap).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -462,9 +469,8 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
   if (flow && (wpos < 0 || wpos >= sync.nwarps)) return;   // no cells: nothing to wait for or publish
   // A cell's routing state and land fractions are read and written each day
   // (mostly L2 hits: the state of the grid is a few MB).  Holding them in
-  // registers for the whole launch instead took ~32 registers per thread, which
-  // the wavefront launch with vertical-balance warps (96 registers per thread)
-  // paid in spills, and measured ~1 % slower on the global grid.
+  // registers for the whole launch instead takes ~32 more of a thread's registers,
+  // which the wavefront launch with vertical-balance warps pays in spills.
   // waiting for outflows, one cell per thread and one day per step (the shape of every
   // single-member FP64 run): what the wait reads of the topology stays in registers,
   // the day's ring values are loaded before the wait and the outflows it has seen are

@@ -178,9 +178,13 @@ __device__ __forceinline__ R lai_nogrowing(int &days, int init, int &status, R l
 
 // Both of the above in FP64, branch-free but for integers: the lanes of a warp are in
 // different states of their leaf area, and four branches of four FP64 operations
-// each cost sixteen, one sum and one multiply-add two (s30: (lmax - lmin) / 30).
+// each cost sixteen, a sum, a product and a multiply-add three. They round as the
+// branches do (span: lmax - lmin), which decides whether a full canopy takes a day's rain
+// to the last bit: a first version with span / 30 on the host did not, and the rounding's
+// 1e-18 km3 of runoff, or none, changed the speed of an empty river and with it the water
+// use that it met, by 1.5e-8 km3.
 __device__ __forceinline__ double lai_fp64(bool warm, int &days, int init, int &status, bool evergreen, bool arid,
-                                           double lmin, double lmax, double s30, double &psum, double prec) {
+                                           double lmin, double lmax, double span, double &psum, double prec) {
   const double p = psum + prec;
   int k = 0;   // days up from lmin (positive) or down from lmax (negative)
   bool from_max = false;
@@ -210,7 +214,7 @@ __device__ __forceinline__ double lai_fp64(bool warm, int &days, int init, int &
       days--;
     }
   }
-  return fma((double)k, s30, from_max ? lmax : lmin);
+  return fma(span * (double)k, 1.0 / 30.0, from_max ? lmax : lmin);
 }
 
 // Where one cell-day's output terms go (FP64): the sums of the day's month, field
@@ -318,7 +322,7 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
   R dailyLai;
   if constexpr (!fp32)
     dailyLai = lai_fp64(Tf > 8.f, days, c.init_days[s], status, (flags & F_EVERGREEN) != 0, arid, c.lai_min[s],
-                        c.lai_max[s], c.lai_s30[s], psum, dailyPrec);
+                        c.lai_max[s], c.lai_span[s], psum, dailyPrec);
   else if (Tf > 8.f)
     dailyLai = lai_growing<R>(days, c.init_days[s], status, (flags & F_EVERGREEN) != 0, arid, c.lai_min[s], c.lai_max[s],
                               psum, dailyPrec);

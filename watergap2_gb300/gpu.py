@@ -506,7 +506,7 @@ class Model:
         return {"vertical_ahead_ms": a.value, "wavefront_ms": b.value, "launch_pairs": n.value}
 
     def step_sync(self, flags: int):
-        """wg_set_step_sync: 0 grid barrier per step, 1 per-warp step flags."""
+        """wg_set_step_sync: 0 waits for outflows or a grid barrier per step, 1 per-warp step flags."""
         self._check(self.lib.wg_set_step_sync(self.h, int(flags)), "set_step_sync")
 
     MONTHLY = {"river_avail": 0, "storage": 1, "min_avail": 2, "max_avail": 3, "cell_runoff": 4, "velocity": 5}
