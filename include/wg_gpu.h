@@ -184,7 +184,8 @@ typedef struct wg_options {
   int32_t days_per_step;   /* days every cell advances per step of the day-pipelined
                               wavefront (1..31; 0 = 1): a run of D days takes
                               ceil(D / days_per_step) + levels - 1 steps.  Results
-                              do not depend on it                                    */
+                              do not depend on it; a whole run (wg_run_days, deferred
+                              days) takes as many up to this as its length is worth  */
   int32_t water_temp;      /* 1: water temperature of the river and every surface water
                               body after each cell's routing (options.calc_wtemp = 1,
                               routing.cpp:4241-4513; fractional routing stays off);
@@ -420,11 +421,12 @@ wg_status wg_get_launch_shape(const wg_ctx *ctx, int32_t *threads, int32_t *bloc
  * integrateWGHM.cpp:414-417). */
 wg_status wg_set_calib_param(wg_ctx *ctx, int32_t k, const double *values);
 
-/* How the wavefront's steps synchronise: 0 = one grid barrier per step (the
- * default); 1 = per-warp step flags, each warp of cells waiting only for the
- * warps that hold its cells' upstream and downstream cells (single-member
- * layout only, WG_ERR_UNSUPPORTED elsewhere).  Results are the same either way;
- * on the global grid the flags measured 3.6 % slower (each warp polls 30-60
+/* How the wavefront's steps synchronise: 0 (the default) = each cell waits for its
+ * upstream cells' outflow of the step before (one member, every cell active, no
+ * GLWD units), or one grid barrier per step (the others); 1 = per-warp step flags,
+ * each warp of cells waiting only for the warps that hold its cells' upstream and
+ * downstream cells (single-member layout only, WG_ERR_UNSUPPORTED elsewhere).
+ * Results are the same either way; the flags are slower (each warp polls 30-60
  * neighbours scattered by the slot order). */
 wg_status wg_set_step_sync(wg_ctx *ctx, int32_t flags);
 
@@ -547,20 +549,22 @@ wg_status wg_get_kernel_times(wg_ctx *ctx, double *vertical_ahead_ms, double *wa
 /* Wavefront steps per launch of wg_run_steps: 1 .. the ring capacity in steps
  * (wg_options.ring_days / days_per_step; half of it with the vertical overlap
  * below); 0 = the default: the ring capacity, or ceil(16 / days_per_step)
- * steps with the overlap.
+ * steps with the overlap.  Launches whose cells wait for outflows have buffer
+ * rows for 64 days and take at most those steps.
  * No counterpart in the reference (it has no day pipelining). */
 wg_status wg_set_chunk_steps(wg_ctx *ctx, int32_t steps);
 int32_t wg_get_chunk_steps(const wg_ctx *ctx);
 
-/* Vertical overlap (one FP64 member with the default launch shape): each
- * wavefront launch of wg_run_steps carries extra warps that run the vertical
+/* Vertical overlap (one FP64 member with the default launch shape): in each
+ * wavefront launch of wg_run_steps the idle warp of every block, further warps
+ * where the block has room, and the routing warps that are done run the vertical
  * balance of the cells without water bodies for the next launch's steps, so the
  * FP64 pipe has that work while the routing warps wait; the first chunk of each
  * call runs its vertical balance in a launch of its own.  On by default where
  * the shape allows it.  enable = 0 switches it off (one vertical-ahead launch
  * before each wavefront launch); WG_ERR_UNSUPPORTED where the shape has no room
- * for the extra warps.  wg_get_vertical_overlap returns the extra warps per
- * block (0: off).  Results are the same bits either way. */
+ * for it.  wg_get_vertical_overlap returns the extra warps per block, at least 1
+ * (0: off).  Results are the same bits either way. */
 wg_status wg_set_vertical_overlap(wg_ctx *ctx, int32_t enable);
 int32_t wg_get_vertical_overlap(const wg_ctx *ctx);
 
@@ -589,7 +593,7 @@ wg_status wg_graph_capture(wg_ctx *ctx, int32_t doy0, int32_t fday0, int32_t nda
 wg_status wg_graph_launch(wg_ctx *ctx);
 
 /* Wait for the context's stream.  WG_ERR_TIMEOUT: a device-side wait (the grid
- * barrier of the wavefront, or a step flag) ran out of its iteration limit; the
+ * barrier of the wavefront, an outflow or a step flag) ran out of its iteration limit; the
  * kernel returned without trapping, the CUDA context stays usable, and the
  * library refuses further results until wg_clear_error (after restoring a
  * state: the run stopped part way). */
@@ -598,7 +602,8 @@ wg_status wg_clear_error(wg_ctx *ctx);
 
 /* Failure-detection test hook: with extra_arrivals > 0 every grid-barrier wait
  * of the following wavefront launches waits for that many arrivals that never
- * come, runs out after its iteration limit (about a second) and reports
+ * come, every wait for an outflow takes none for one, and both run out after their
+ * iteration limits (about a second) and report
  * WG_ERR_TIMEOUT through wg_synchronize.  0 (the default) for normal runs. */
 wg_status wg_set_barrier_test(wg_ctx *ctx, int32_t extra_arrivals);
 
