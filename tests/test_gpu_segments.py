@@ -1,0 +1,103 @@
+"""Parts of a run: steps t_begin > 0 from a graph, run again on the state they find, and
+beside a change of what the steps wait for, against the step flags, whose calls keep
+their outflows in the same two rows throughout."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+DOY0, ND = 330, 90
+
+
+def _model(temp=False, flags=False, kd=1, **kw):
+    from watergap2_gb300 import synthetic as sy
+    from watergap2_gb300.gpu import Model
+    region = sy.region_small_swb(seed=5, ny=17, nx=31, river_velo_opt=2)
+    P, T, S = sy.forcing(region, ND, seed=4, doy0=DOY0)
+    m = Model(region, max_days=ND, days_per_step=kd, stations=np.arange(region.ncell), water_temp=temp, **kw)
+    if temp:
+        m.set_water_temp_inputs(np.full(region.ncell, 9., np.float32))
+        m.upload_longwave(0, 250. + T)
+    if flags:
+        m.vertical_overlap(False)
+        m.step_sync(1)
+    m.upload_forcing(0, P, T, S)
+    return m
+
+
+def _all(m, temp):
+    s = m.get_state()
+    out = [m.discharge(0, ND)] + [np.asarray(s[k]) for k in sorted(s)]
+    if temp:
+        out += [*m.water_temp(), m.river_temp(0, ND)]
+    return out
+
+
+def _same(a, b):
+    assert np.isfinite(a[0]).all() and a[0].max() > 0
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("kd", [1, 5])
+@pytest.mark.parametrize("temp", [False, True])
+def test_graph_of_a_later_part(temp, kd):
+    """Captured before the steps that lead to it have run, and before a graph of a
+    whole run or a change of the waits would have told it anything."""
+    ref = _model(temp, True, kd)
+    total = ref.num_steps(ND)
+    a, b = total // 4, total // 2
+    ref.run_steps(DOY0, 0, ND, 0, total)
+    m = _model(temp, False, kd)
+    m.graph_capture(DOY0, 0, ND, a, b)
+    m.run_steps(DOY0, 0, ND, 0, a)
+    m.graph_launch()
+    m.run_steps(DOY0, 0, ND, b, total)
+    _same(_all(m, temp), _all(ref, temp))
+
+
+@pytest.mark.parametrize("kd", [1, 5])
+@pytest.mark.parametrize("temp", [False, True])
+def test_steps_run_again(temp, kd):
+    """A part longer than the rows of the waits, to the end of the run and into it."""
+    got = []
+    for flags in (True, False):
+        m = _model(temp, flags, kd)
+        total = m.num_steps(ND)
+        m.run_steps(DOY0, 0, ND, 0, 20 // kd)
+        m.save_snapshot()
+        for end in (total, total - 3, total // 2):
+            for _ in range(2):
+                m.run_steps(DOY0, 0, ND, 20 // kd, end)
+        out = _all(m, temp)
+        m.restore_snapshot()
+        if not flags:
+            m.graph_capture(DOY0, 0, ND, 20 // kd, total)
+        for _ in range(2):
+            m.run_steps(DOY0, 0, ND, 20 // kd, total) if flags else m.graph_launch()
+        got.append(out + _all(m, temp))
+    _same(*got)
+
+
+def test_waits_changed_between_the_steps():
+    ref = _model(flags=True)
+    total = ref.num_steps(ND)
+    ref.run_steps(DOY0, 0, ND, 0, total)
+    m = _model()
+    cells = m.region.ncell
+    cuts = [0, 1, 2, 7, 30, 31, 80, total]
+    for k, (a, b) in enumerate(zip(cuts, cuts[1:])):
+        m.step_sync(k % 3 == 1)
+        m.set_active_cells(np.ones(cells) if k % 3 == 2 else None)
+        m.run_steps(DOY0, 0, ND, a, b)
+    _same(_all(m, False), _all(ref, False))
+
+
+def test_autotune_on_later_steps_after_a_shorter_run():
+    ref = _model(flags=True)
+    ref.run_days(DOY0, 0, 40)
+    m = _model()
+    m.run_days(DOY0, 0, 40)
+    m.autotune(DOY0, 0, ND, 70, 30)
+    s, r = m.get_state(), ref.get_state()
+    for k in s:
+        assert np.array_equal(s[k], r[k])

@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -1905,6 +1906,42 @@ wg_status wg_step_routing(wg_ctx *ctx, int32_t doy, int32_t oday) {
 
 }  // extern "C"
 
+// How the wavefront's steps wait for one another: for the outflows themselves where
+// every cell runs, else at a grid barrier.  Between two calls a run's outflows lie in
+// the two rows of the barrier whatever the calls wait for, so that a call may follow
+// any other (a graph captured earlier, one under another mask or wg_set_step_sync, the
+// same steps again); the rows of the waits hold nothing from one call to the next.
+struct StepSync { DevSync sync; double *outq; DevWaterTemp wt; };
+static StepSync step_sync(wg_ctx *ctx, int kd, bool one_step = false) {
+  StepSync r{ctx->sync, ctx->outq, ctx->wt};
+  r.sync.rows = 2;
+  r.sync.data = ctx->outq_days > 0 && !ctx->sync.flow && !ctx->cells_skipped() && !one_step;
+  r.sync.keep_from = INT_MAX;
+  if (r.sync.data) {
+    const size_t skip = (size_t)2 * ctx->days_per_step * ctx->nstate();
+    r.sync.kept = r.outq;
+    r.sync.kept_t = r.wt.outt;
+    r.outq += skip;
+    if (r.wt.outt) r.wt.outt += skip;
+    r.sync.rows = ctx->outq_days / kd;
+  }
+  return r;
+}
+
+// The two rows at a call of steps [t_b, t_e): what the step before left goes to the row
+// that step t_b reads, and the launches write them from keep_from on. Each step
+// overwrites its parity's row, so that takes the call's last two steps and those from
+// which on the first cells are done with the run. A whole run leaves them as they are.
+// (A call of one step waits for nothing and works in the two rows themselves.)
+static cudaError_t kept_rows(wg_ctx *ctx, StepSync &ss, int kd, int ndays, int t_b, int t_e) {
+  if (!ss.sync.data || (t_b == 0 && t_e == ctx->total_steps(ndays, kd))) return cudaSuccess;
+  ss.sync.keep_from = std::min(t_e - 2, (ndays + kd - 1) / kd - 3);
+  if (t_b == 0) return cudaSuccess;
+  const size_t row = (size_t)kd * ctx->nstate(), to = (t_b - 1) % ss.sync.rows * row, from = ((t_b - 1) & 1) * row;
+  return launch_fetch_row(ss.outq + to, ss.sync.kept + from, ss.wt.enabled ? ss.wt.outt + to : nullptr,
+                          ss.wt.enabled ? ss.sync.kept_t + from : nullptr, row, ctx->stream);
+}
+
 // Steps [t_b, t_e) of the day-pipelined wavefront of a run of ndays days, in
 // chunks: the vertical balance of the cells without water bodies runs ahead of
 // each chunk's routing wavefront (one cooperative launch).  Without the overlap it
@@ -1912,34 +1949,15 @@ wg_status wg_step_routing(wg_ctx *ctx, int32_t doy, int32_t oday) {
 // wavefront launch carries warps that compute the next chunk's, so the FP64 pipe
 // has their work while the routing warps wait on loads and step barriers.  Every
 // call ends with the vertical state exactly at step t_e either way.
-// How the wavefront's steps wait for one another: for the outflows themselves where
-// every cell runs, else at a grid barrier.  A run keeps the buffer that it began with.
-struct StepSync { DevSync sync; double *outq; DevWaterTemp wt; };
-static StepSync step_sync(wg_ctx *ctx, int kd, bool data) {
-  StepSync r{ctx->sync, ctx->outq, ctx->wt};
-  r.sync.rows = 2;
-  r.sync.data = 0;
-  if (data) {
-    const size_t skip = (size_t)2 * ctx->days_per_step * ctx->nstate();
-    r.outq += skip;
-    if (r.wt.outt) r.wt.outt += skip;
-    r.sync.rows = ctx->outq_days / kd;
-    r.sync.data = !ctx->cells_skipped();
-  }
-  return r;
-}
-static bool data_sync_possible(const wg_ctx *ctx) {
-  return ctx->outq_days > 0 && !ctx->sync.flow && !ctx->cells_skipped();
-}
-
 template <class R>
 static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevStateT<R> &s, const DevVertT<R> &v,
                                 DevRingT<R> ring, int kd, int doy0, int fday0, int oday0, int ndays, int t_b,
                                 int t_e) {
   ring.days_per_step = kd;
   const bool ov = ctx->overlap();
-  if (t_b == 0) ctx->run_data = data_sync_possible(ctx);
-  const StepSync ss = step_sync(ctx, kd, ctx->run_data);
+  StepSync ss = step_sync(ctx, kd, t_e - t_b == 1);
+  const cudaError_t ke = kept_rows(ctx, ss, kd, ndays, t_b, t_e);
+  if (ke != cudaSuccess) return cuda_fail(ctx, ke, "run_steps");
   // (waiting for outflows, a launch's steps have rows of their own beside the one before)
   const int chunk = ss.sync.data ? std::min(ctx->eff_chunk(kd), ss.sync.rows - 1) : ctx->eff_chunk(kd);
   if (ctx->ens_overlap && ctx->members > 1 && ctx->va_stream) {
@@ -2048,7 +2066,7 @@ static wg_status routing_now(wg_ctx *ctx, int doy, int oday) {
   cudaSetDevice(ctx->device);
   join_uploads(ctx);
   ctx->launches++;
-  StepSync ss = step_sync(ctx, 1, data_sync_possible(ctx));
+  StepSync ss = step_sync(ctx, 1);
   if (ss.sync.data) ss.sync.rows = 1;   // one day: a cell's outflow is written once
   cudaError_t e = ctx->precision == 0
                       ? launch_pipeline(false, ctx->cd, ctx->sd, ctx->vd, ctx->forcing, ctx->mem, ctx->balance,

@@ -83,11 +83,11 @@ struct wg_ctx {
   bool has_kc = false;                     // the region gave the LCT crop coefficients
   std::vector<double> cell_area, cell_cont;   // cell order: area [km2], continental share [%] as raised
   double *daily_storage_buf = nullptr;     // wg_record_daily_storages (context allocation)
-  // the outflow buffer: two steps of days for the wavefront with a grid barrier, then
-  // outq_days days of rows for the one that waits for the outflows themselves
-  // (DevSync::data; 0: none), the water temperature's outt likewise
+  // the outflow buffer: two steps of days for the wavefront with a grid barrier, which
+  // also hold a run's outflows between calls, then outq_days days of rows for the one
+  // that waits for the outflows themselves (DevSync::data; 0: none; nothing of them is
+  // kept from one call to the next), the water temperature's outt likewise
   int outq_days = 0;
-  bool run_data = false;                   // which of the two the run in progress uses
   size_t outq_rows() const { return (size_t)2 * days_per_step + outq_days; }
   bool cells_skipped() const { return (precision == 0 ? cd.active : cf.active) != nullptr; }
   double *outq = nullptr, *qst = nullptr, *vol0 = nullptr, *partial = nullptr;

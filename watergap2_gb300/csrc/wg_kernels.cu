@@ -738,11 +738,15 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
           }
           if (ENS) q_now[si] = (double)tv;
           else st_outflow(q_now + si, (double)tv);
+          const bool keep = FUSED && !ENS && t >= sync.keep_from;
+          const size_t kept_at = ((size_t)(t & 1) * kd + kk) * N + si;
+          if (keep) st_outflow(sync.kept + kept_at, (double)tv);
           if constexpr (WT) {
             // a cell without continental area keeps the reference's initial 15 degrees (routing.cpp:174)
             const double tr = nocont ? 15. : wtd.river((double)rs.river, (double)c.rlen[s], (double)c.cfa[s],
                                                        (double)o.owpet);
             st_outflow(t_now0 + (size_t)kk * N + si, tr);
+            if (keep) st_outflow(sync.kept_t + kept_at, tr);
             const int stw = c.station[s];
             if (stw >= 0) wtp.qst_t[(size_t)(oday0 + d) * c.nstation + stw] = tr;
           }
@@ -1040,6 +1044,20 @@ cudaError_t launch_rows(const double *src, const double *land, double *out, cons
   if (total == 0) return cudaSuccess;
   k_rows<<<(unsigned)std::min<size_t>((total + 255) / 256, 152 * 32), 256, 0, st>>>(src, land, out, slot_of_cell, n,
                                                                                  members, rows, no_inf);
+  return cudaGetLastError();
+}
+
+// One row of outflows (2.7 MB on the global grid at five days per step), before a call
+// that goes on with a run: a launch costs 3 us of the stream where a copy costs 9.
+__global__ void __launch_bounds__(256) k_fetch_row(double *dst, const double *src, double *dst_t, const double *src_t, size_t n) {
+  double *d = blockIdx.y ? dst_t : dst;
+  const double *s = blockIdx.y ? src_t : src;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) d[i] = s[i];
+}
+
+cudaError_t launch_fetch_row(double *dst, const double *src, double *dst_t, const double *src_t, size_t n, cudaStream_t st) {
+  const dim3 grid((unsigned)std::min<size_t>((n + 255) / 256, 152 * 32), dst_t ? 2 : 1);
+  k_fetch_row<<<grid, 256, 0, st>>>(dst, src, dst_t, src_t, n);
   return cudaGetLastError();
 }
 

@@ -77,6 +77,8 @@ cudaError_t launch_pipeline(bool fused, const DevCellsT<R> &c, const DevStateT<R
                             int t_b, int t_e, int blocks, int threads, const WarpLayout &lay, const DevMonthly &mon,
                             const DevVaWork &vw, const DevWaterTemp &wtp, const DevWaterUse &wu, cudaStream_t st);
 cudaError_t launch_fill(double *p, size_t n, double v, cudaStream_t st);
+// n doubles from src to dst and, where there are any, from src_t to dst_t
+cudaError_t launch_fetch_row(double *dst, const double *src, double *dst_t, const double *src_t, size_t n, cudaStream_t st);
 template <class R>
 cudaError_t launch_vertical_ahead(const DevCellsT<R> &c, const DevStateT<R> &s, const DevForcing &f,
                                   const DevMembers &mem, const DevBalance &b, const DevRingT<R> &ring, int doy0,

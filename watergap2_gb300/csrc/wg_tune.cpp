@@ -18,14 +18,13 @@
 using namespace wg;
 
 // Device copy of everything a run mutates: the state arrays, the snow bands,
-// the two-slot outflow buffer of the wavefront and the balance accumulators.
+// the two steps of outflows that lie between calls and the balance accumulators.
 // (The ring of vertical outputs holds nothing between calls: each chunk's
 // vertical-ahead launch fills exactly the days its wavefront launch reads.)
 struct Snapshot {
   std::vector<std::pair<void *, size_t>> fields;   // (device array, bytes)
   char *buf = nullptr;
   size_t bytes = 0;
-  bool run_data = false;                           // wg_ctx::run_data
 };
 
 namespace {
@@ -46,13 +45,13 @@ void list_fields(wg_ctx *ctx, const DevStateT<R> &s, Snapshot &sn) {
   WG_STATE_I(X)
 #undef X
   sn.fields.push_back({(void *)s.snow_band, N * ctx->nband * sizeof(R)});
-  sn.fields.push_back({(void *)ctx->outq, ctx->outq_rows() * N * sizeof(double)});
+  sn.fields.push_back({(void *)ctx->outq, 2 * (size_t)ctx->days_per_step * N * sizeof(double)});
   if (ctx->balance.enabled) sn.fields.push_back({(void *)ctx->balance.acc, WG_BALANCE_ARRAYS * N * sizeof(double)});
   if (ctx->wu.enabled) sn.fields.push_back({(void *)ctx->wu.st, (size_t)wg::WU_NSTATE * N * sizeof(double)});
   if (ctx->wt.enabled) {
     sn.fields.push_back({(void *)ctx->wt.temp, 6 * N * sizeof(double)});
     sn.fields.push_back({(void *)ctx->wt.ice, 6 * N * sizeof(double)});
-    sn.fields.push_back({(void *)ctx->wt.outt, ctx->outq_rows() * N * sizeof(double)});
+    sn.fields.push_back({(void *)ctx->wt.outt, 2 * (size_t)ctx->days_per_step * N * sizeof(double)});
   }
 }
 
@@ -69,7 +68,6 @@ wg_status snapshot_save(wg_ctx *ctx) {
     }
     ctx->snap = sn;
   }
-  ctx->snap->run_data = ctx->run_data;
   size_t off = 0;
   for (auto &f : ctx->snap->fields) {
     cudaError_t e = cudaMemcpyAsync(ctx->snap->buf + off, f.first, f.second, cudaMemcpyDeviceToDevice, ctx->stream);
@@ -81,7 +79,6 @@ wg_status snapshot_save(wg_ctx *ctx) {
 
 wg_status snapshot_restore(wg_ctx *ctx) {
   if (!ctx->snap) return WG_ERR_INVALID;
-  ctx->run_data = ctx->snap->run_data;
   size_t off = 0;
   for (auto &f : ctx->snap->fields) {
     cudaError_t e = cudaMemcpyAsync(f.first, ctx->snap->buf + off, f.second, cudaMemcpyDeviceToDevice, ctx->stream);
