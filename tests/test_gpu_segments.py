@@ -8,11 +8,16 @@ pytestmark = pytest.mark.gpu
 DOY0, ND = 330, 90
 
 
+def _forcing(region):
+    from watergap2_gb300 import synthetic as sy
+    return sy.forcing(region, ND, seed=4, doy0=DOY0)
+
+
 def _model(temp=False, flags=False, kd=1, **kw):
     from watergap2_gb300 import synthetic as sy
     from watergap2_gb300.gpu import Model
     region = sy.region_small_swb(seed=5, ny=17, nx=31, river_velo_opt=2)
-    P, T, S = sy.forcing(region, ND, seed=4, doy0=DOY0)
+    P, T, S = _forcing(region)
     m = Model(region, max_days=ND, days_per_step=kd, stations=np.arange(region.ncell), water_temp=temp, **kw)
     if temp:
         m.set_water_temp_inputs(np.full(region.ncell, 9., np.float32))
@@ -101,3 +106,64 @@ def test_autotune_on_later_steps_after_a_shorter_run():
     s, r = m.get_state(), ref.get_state()
     for k in s:
         assert np.array_equal(s[k], r[k])
+
+
+def _above(region, x):
+    """The cells above cell x."""
+    up = np.zeros(region.ncell, bool)
+    for i in region.rout_order[::-1]:
+        d = region.downstream[i]
+        up[i] = d >= 0 and (d == x or up[d])
+    return up
+
+
+def _cell_with_upstream(region):
+    n = [_above(region, x).sum() for x in range(region.ncell)]
+    return int(np.argsort(n)[-3])
+
+
+@pytest.mark.parametrize("restored", [False, True])
+def test_a_skipped_cell_has_no_outflow(restored):
+    """Days routed before the mask leave nothing behind for the cells below it: as in
+    the region whose river is cut there."""
+    import copy
+    from watergap2_gb300.gpu import Model
+    m = _model()
+    x = _cell_with_upstream(m.region)
+    skip = _above(m.region, x)
+    m.set_active_cells(np.ones(m.region.ncell))   # routed with a grid barrier per step
+    m.run_days(DOY0, 0, 20)
+    s = m.get_state()
+    if restored:
+        m.save_snapshot()
+    m.set_active_cells(~skip)
+    if restored:
+        m.restore_snapshot()
+    m.run_days((DOY0 - 1 + 20) % 365 + 1, 20, 30)
+
+    cut = copy.deepcopy(m.region)
+    cut.arrays["downstream"][skip & (cut.downstream == x)] = -1
+    P, T, S = _forcing(m.region)
+    r = Model(cut, max_days=ND, stations=np.arange(cut.ncell))
+    r.upload_forcing(0, P, T, S)
+    r.set_state(s)
+    r.set_active_cells(~skip)
+    r.run_days((DOY0 - 1 + 20) % 365 + 1, 20, 30)
+    a, b = m.discharge(20, 30)[:, ~skip], r.discharge(20, 30)[:, ~skip]
+    assert a.max() > 0 and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("temp", [False, True])
+def test_a_mask_set_in_mid_run(temp):
+    got = []
+    for flags in (True, False):
+        m = _model(temp, flags)
+        total = m.num_steps(ND)
+        m.run_steps(DOY0, 0, ND, 0, 70)
+        skip = _above(m.region, _cell_with_upstream(m.region))
+        m.set_active_cells(~skip)
+        m.run_steps(DOY0, 0, ND, 70, 80)
+        m.set_active_cells(None)
+        m.run_steps(DOY0, 0, ND, 80, total)
+        got.append(_all(m, temp))
+    _same(*got)

@@ -2661,7 +2661,7 @@ wg_status wg_set_active_cells(wg_ctx *ctx, const uint8_t *active) {
   }
   ctx->cd.active = dev;
   ctx->cf.active = dev;
-  return WG_OK;
+  return cuda_fail(ctx, ctx->clear_skipped(), "set_active_cells");
 }
 
 wg_status wg_set_calib_param(wg_ctx *ctx, int32_t k, const double *values) {

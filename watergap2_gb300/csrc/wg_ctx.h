@@ -89,6 +89,13 @@ struct wg_ctx {
   // kept from one call to the next), the water temperature's outt likewise
   int outq_days = 0;
   size_t outq_rows() const { return (size_t)2 * days_per_step + outq_days; }
+  // a cell that is skipped produces no outflow: the rows between calls, whose layout
+  // (one day per step or more) a call decides, at a new mask and after a restore
+  cudaError_t clear_skipped() {
+    return cells_skipped() ? wg::launch_clear_skipped(outq, wt.enabled ? wt.outt : nullptr, d_active, n, members,
+                                                      2 * days_per_step, stream)
+                           : cudaSuccess;
+  }
   bool cells_skipped() const { return (precision == 0 ? cd.active : cf.active) != nullptr; }
   double *outq = nullptr, *qst = nullptr, *vol0 = nullptr, *partial = nullptr;
   float *staging = nullptr;

@@ -1047,6 +1047,23 @@ cudaError_t launch_rows(const double *src, const double *land, double *out, cons
   return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256) k_clear_skipped(double *rows, double *rows_t, const uint8_t *__restrict__ active,
+                                                       int members, size_t row, size_t total) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    if (active[i % row / members]) continue;
+    rows[i] = 0.;
+    if (rows_t) rows_t[i] = 0.;
+  }
+}
+
+cudaError_t launch_clear_skipped(double *rows, double *rows_t, const uint8_t *active, int n, int members, int nrows,
+                                 cudaStream_t st) {
+  const size_t row = (size_t)n * members, total = row * nrows;
+  k_clear_skipped<<<(unsigned)std::min<size_t>((total + 255) / 256, 152 * 32), 256, 0, st>>>(rows, rows_t, active, members,
+                                                                                           row, total);
+  return cudaGetLastError();
+}
+
 // One row of outflows (2.7 MB on the global grid at five days per step), before a call
 // that goes on with a run: a launch costs 3 us of the stream where a copy costs 9.
 __global__ void __launch_bounds__(256) k_fetch_row(double *dst, const double *src, double *dst_t, const double *src_t, size_t n) {

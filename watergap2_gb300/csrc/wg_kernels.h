@@ -77,6 +77,10 @@ cudaError_t launch_pipeline(bool fused, const DevCellsT<R> &c, const DevStateT<R
                             int t_b, int t_e, int blocks, int threads, const WarpLayout &lay, const DevMonthly &mon,
                             const DevVaWork &vw, const DevWaterTemp &wtp, const DevWaterUse &wu, cudaStream_t st);
 cudaError_t launch_fill(double *p, size_t n, double v, cudaStream_t st);
+// no outflow (and river temperature, rows_t null: none) of the cells that active leaves
+// out, in nrows rows of n cells x members
+cudaError_t launch_clear_skipped(double *rows, double *rows_t, const uint8_t *active, int n, int members, int nrows,
+                                 cudaStream_t st);
 // n doubles from src to dst and, where there are any, from src_t to dst_t
 cudaError_t launch_fetch_row(double *dst, const double *src, double *dst_t, const double *src_t, size_t n, cudaStream_t st);
 template <class R>

@@ -85,7 +85,7 @@ wg_status snapshot_restore(wg_ctx *ctx) {
     if (e != cudaSuccess) return fail(ctx, e, "restore");
     off += (f.second + 255) / 256 * 256;
   }
-  return WG_OK;
+  return fail(ctx, ctx->clear_skipped(), "restore");
 }
 
 }  // namespace
