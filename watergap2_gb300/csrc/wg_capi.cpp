@@ -397,17 +397,18 @@ size_t states_per_thread(const wg_ctx *ctx) {
 }
 
 // An ensemble's launches for the context's block size. Wavefront: blocks are joined up to
-// the kernel's 512 threads where that still fills the GPU -- the more warps share a
-// block's states, the more evenly a step's work spreads over them; fewer states than
-// that are spread over as many SMs as there are blocks. Vertical balance ahead, whose
+// the kernel's 1,024 threads where that fills the GPU as they did -- the more warps share
+// a block's states, the more evenly a step's work spreads over them; fewer states than
+// that are spread over as many SMs as there are blocks. (The launch is cooperative: no
+// more joined blocks than the GPU holds. Ten blocks of 96 threads an SM make one of 960;
+// eight, 768, would have been 190 blocks for 152 SMs.) Vertical balance ahead, whose
 // threads share nothing: on the second stream as many blocks as the GPU holds, by
 // itself one (cell, member) per thread, so that blocks start as SMs come free.
 void set_ensemble_shape(wg_ctx *ctx) {
   constexpr int kMost = PipeBounds<float, true>::threads;
-  ctx->layout.join = 1;
-  while (ctx->threads * ctx->layout.join * 2 <= kMost) ctx->layout.join *= 2;
+  ctx->layout.join = kMost / ctx->threads;
   if (states_per_thread(ctx) < 1 ||
-      ctx->blocks_fused / ctx->layout.join < pipeline_max_blocks<float>(true, true, ctx->threads * ctx->layout.join))
+      ctx->blocks_fused / ctx->layout.join != pipeline_max_blocks<float>(true, true, ctx->threads * ctx->layout.join))
     ctx->layout.join = 1;
   ctx->threads_va = std::min(ctx->threads, 64);
   const size_t need = std::min<size_t>((ctx->nstate() + ctx->threads_va - 1) / ctx->threads_va, (size_t)1 << 30);
