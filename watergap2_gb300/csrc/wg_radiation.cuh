@@ -9,8 +9,11 @@
 // In FP64 they were 27 multiplications and additions, two exponentials and three
 // reciprocals of every cell-day, a fifth of the vertical balance's FP64-pipe
 // time.  T is a float, so here it is one 64-bit integer; products are 64 x 64-bit
-// high parts at constant scales, and only the three results are rounded to double
-// (relative error below 2^-52; the FP64 chain rounded some twenty times).
+// high parts at constant scales, and only the three results are rounded to double:
+// rlh and apt to a relative error below 2^-52, where the FP64 chain rounded some twenty
+// times; lwt to 2^-51 of 0.281 sigma (T + 273.2)^4 / latent heat, an absolute error, since
+// its emissivity 0.261 exp(-0.000777 T^2) - 0.02 changes sign near |T| = 57.5 C (in FP64
+// the same subtraction cancels there).
 #pragma once
 #include <stdint.h>
 
