@@ -562,7 +562,9 @@ __device__ __forceinline__ void vertical_cell(const DevCellsT<R> &c, int s, R ga
     if constexpr (fp32) {
       effPrec *= invB;
     } else {
-      if (!cmp::is_zero(prec_to_soil)) effPrec = n_rainfall == B ? prec_to_soil : (double)n_rainfall * invB * prec_to_soil;
+      // (no band with rain: nothing, of infinite precipitation too)
+      if (n_rainfall && !cmp::is_zero(prec_to_soil))
+        effPrec = n_rainfall == B ? prec_to_soil : (double)n_rainfall * invB * prec_to_soil;
       if (!cmp::is_zero(out_melt)) effPrec += out_melt * invB;
     }
     if (any_snow) {   // else all zero
