@@ -1161,9 +1161,13 @@ cudaError_t launch_vertical_ahead(const DevCellsT<R> &c, const DevStateT<R> &s, 
 template <class R>
 cudaError_t launch_pet(const DevCellsT<R> &c, const DevForcing &f, const DevRingT<R> &ring, int doy0, int fday0,
                        int ndays, int t_b, int t_e, cudaStream_t st) {
-  const long long days = (long long)ring.days_per_step * (t_e - t_b);
-  const dim3 grid((unsigned)((c.n + 255) / 256), (unsigned)((days + kPetDays - 1) / kPetDays));
-  k_pet<R><<<grid, 256, 0, st>>>(c, f, ring, doy0, fday0, ndays, t_b, t_e);
+  const int most = 65535 * kPetDays / ring.days_per_step;   // steps that the grid's second dimension holds
+  for (int a = t_b; a < t_e; a += most) {
+    const int b = std::min(t_e, a + most);
+    const long long days = (long long)ring.days_per_step * (b - a);
+    const dim3 grid((unsigned)((c.n + 255) / 256), (unsigned)((days + kPetDays - 1) / kPetDays));
+    k_pet<R><<<grid, 256, 0, st>>>(c, f, ring, doy0, fday0, ndays, a, b);
+  }
   return cudaGetLastError();
 }
 
