@@ -180,7 +180,9 @@ typedef struct wg_options {
                            /* wavefront where the states fill the GPU)                 */
   int32_t ring_days;       /* days of vertical outputs buffered between the vertical
                               balance run ahead and routing; 0 = as many as fit in 8 GB
-                              or an eighth of the free device memory, the smaller */
+                              (ensembles 24) or an eighth of the free device memory, the
+                              smaller, and up to half as much for their potential
+                              evapotranspiration                                      */
   int32_t days_per_step;   /* days every cell advances per step of the day-pipelined
                               wavefront (1..31; 0 = 1): a run of D days takes
                               ceil(D / days_per_step) + levels - 1 steps.  Results

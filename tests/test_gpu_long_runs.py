@@ -19,3 +19,12 @@ def test_evaporation_of_more_days_than_a_grid_holds():
         q.append(m.discharge(nd - 365, 365))
         m.close()
     assert q[0].max() > 0 and np.array_equal(*q)
+
+
+def test_the_ring_holds_as_many_days_as_its_memory():
+    """8 GB of runoff and recharge; a launch may take half of them."""
+    from watergap2_gb300 import synthetic as sy
+    from watergap2_gb300.gpu import Model
+    m = Model(sy.region_64x64(), max_days=100_000)
+    assert m.vertical_overlap() > 0
+    assert m.chunk_steps(50_000) == 50_000

@@ -1383,10 +1383,11 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t)16 << 30;
     // (ensembles: 24 GB, so that the ring holds two chunks of the stream overlap)
     const size_t ring_bytes = std::min<size_t>((size_t)(ctx->members > 1 ? 24 : 8) << 30, free_b / 8);
-    // per day: surface runoff and recharge of every state, the PETs of every cell (with
-    // one member two of the three wait in the slots that runoff and recharge overwrite)
+    // per day: surface runoff and recharge of every state (with one member two of the
+    // cells' three PETs wait in the slots that runoff and recharge overwrite; the third,
+    // and an ensemble's three, come on top: half as much again and less)
     const bool ens_ring = ctx->members > 1;
-    const size_t budget = opt->ring_days > 0 ? (size_t)opt->ring_days : ring_bytes / (elem * (2 * N + (ens_ring ? 3 : 1) * (size_t)n));
+    const size_t budget = opt->ring_days > 0 ? (size_t)opt->ring_days : ring_bytes / (2 * elem * N);
     const int ring = (int)std::max<size_t>(std::max(8, 2 * ctx->days_per_step),
                                            std::min<size_t>(budget, (size_t)ctx->max_days));
     ctx->rd.days_per_step = ctx->rf.days_per_step = ctx->days_per_step;
