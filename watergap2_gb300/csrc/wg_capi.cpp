@@ -2001,13 +2001,17 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
   }
   DevVaWork vw{};
   vw.next = ctx->va_next;
-  int pet_end = t_b;   // the ring holds the PET of the steps before pet_end
-  for (int a = t_b; a < t_e; a += chunk) {
-    const int b = std::min(t_e, a + chunk);
+  int pet_end = t_b, va_end = t_b;   // the ring holds the PET and the runoff of the steps before them
+  for (int a = t_b, b; a < t_e; a = b) {
+    // the vertical balance of all the steps that the ring holds or the chunk length asks
+    // for, however few of them a wavefront launch has rows for
+    const bool va = ov ? a == t_b : a >= va_end;
+    if (va) va_end = std::min(t_e, a + (ov ? chunk : ctx->eff_chunk(kd)));
+    b = std::min(ov ? t_e : va_end, a + chunk);
     cudaEvent_t *ev = ctx->timing ? ctx->timing_events() : nullptr;
     if (ev) cudaEventRecord(ev[0], ctx->stream);
     cudaError_t e = cudaSuccess;
-    if (pet_end < std::min(t_e, ov ? b + chunk : b)) {
+    if (pet_end < (ov ? std::min(t_e, b + chunk) : va_end)) {
       // as many steps as the ring holds from this chunk on (a whole call where it
       // fits); the slots it overwrites were read by the launches before
       const int to = std::min(t_e, a + ctx->max_chunk(kd));
@@ -2015,8 +2019,8 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
       if (e != cudaSuccess) return cuda_fail(ctx, e, "run_steps");
       pet_end = to;
     }
-    if (!ov || a == t_b) {
-      e = launch_vertical_ahead(c, s, ctx->forcing, ctx->mem, ctx->balance, ring, doy0, fday0, ndays, a, b,
+    if (va) {
+      e = launch_vertical_ahead(c, s, ctx->forcing, ctx->mem, ctx->balance, ring, doy0, fday0, ndays, a, va_end,
                                 ctx->members > 1 ? ctx->blocks_va_alone : ctx->blocks_fused,
                                 ctx->members > 1 ? ctx->threads_va : ctx->threads, ctx->stream, ctx->mon, oday0,
                                 states_per_thread(ctx) >= 8);
