@@ -552,7 +552,9 @@ wg_status wg_get_kernel_times(wg_ctx *ctx, double *vertical_ahead_ms, double *wa
  * (wg_options.ring_days / days_per_step; half of it with the vertical overlap
  * below); 0 = the default: the ring capacity, or ceil(16 / days_per_step)
  * steps with the overlap.  Launches whose cells wait for outflows have buffer
- * rows for 64 days and take at most those steps.
+ * rows for 64 days or eight steps, the longer, and take at most those steps (the rows
+ * hold a double per cell and day, two with the water temperature: 35 MB for the global
+ * half-degree grid).
  * No counterpart in the reference (it has no day pipelining). */
 wg_status wg_set_chunk_steps(wg_ctx *ctx, int32_t steps);
 int32_t wg_get_chunk_steps(const wg_ctx *ctx);

@@ -35,3 +35,17 @@ def test_same_bits_as_a_grid_barrier(precision, temp, kd, chunk):
     assert np.isfinite(got[0][0]).all() and got[0][0].max() > 0
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+def test_long_steps_share_launches():
+    """Steps of 31 days: eight to a launch, not one."""
+    from watergap2_gb300 import synthetic as sy
+    from watergap2_gb300.gpu import Model
+    region, nd = sy.region_64x64(size=9), 31 * 40
+    P, T, S = sy.forcing(region, nd, seed=4)
+    m = Model(region, max_days=nd, days_per_step=31, precision="fp32")
+    m.upload_forcing(0, P, T, S)
+    total, before = m.num_steps(nd), m.launch_count
+    m.run_steps(1, 0, nd, 0, total)
+    m.synchronize()
+    assert total >= 40 and m.launch_count - before <= 2 * -(-total // 8)

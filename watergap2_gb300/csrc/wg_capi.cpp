@@ -380,8 +380,10 @@ void join_uploads(wg_ctx *ctx) {
 }
 
 // Days of rows in the outflow buffer of the wavefront that waits for outflows: its
-// launches run up to that many days less one step (the default chunk is 16 days).
-constexpr int kDataDays = 65;
+// launches run up to that many days less one step (the default chunk is 16 days), and
+// eight steps where those are long (with one or two to a launch, 550,000 FP32 cells, 200
+// days in steps of 31 95.9 ms, of 17 55.2; with eight 83.0 and 49.6).
+constexpr int kDataDays = 65, kDataSteps = 9;
 
 bool valid_block_threads(int threads, int precision, int members) {
   const int mx = members > 1 ? 128
@@ -1424,7 +1426,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
   ctx->staging_bytes = std::max<size_t>((size_t)ctx->staging_days * sizeof(float), 30 * sizeof(double)) * n;
   ctx->staging = ctx->alloc<float>(ctx->staging_bytes / sizeof(float));
   // (one member; with GLWD units a cell's upstream cells may be further upstream in steps)
-  ctx->outq_days = ctx->members == 1 && !ctx->glwd.on ? std::max(kDataDays, 2 * ctx->days_per_step) : 0;
+  ctx->outq_days = ctx->members == 1 && !ctx->glwd.on ? std::max(kDataDays, kDataSteps * ctx->days_per_step) : 0;
   ctx->outq = ctx->alloc<double>(ctx->outq_rows() * N);
   ctx->qst = ctx->alloc<double>((size_t)ctx->max_days * std::max(1, ctx->nstation) * ctx->members);
   ctx->balance.enabled = opt->record_balance ? 1 : 0;
