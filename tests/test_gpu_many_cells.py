@@ -49,3 +49,22 @@ def test_long_steps_share_launches():
     m.run_steps(1, 0, nd, 0, total)
     m.synchronize()
     assert total >= 40 and m.launch_count - before <= 2 * -(-total // 8)
+
+
+@pytest.mark.parametrize("members", [1, 3])
+def test_long_runs_that_gain_nothing_from_longer_steps_take_days(members):
+    """As many launches with up to four days per step as with one."""
+    from watergap2_gb300 import synthetic as sy
+    from watergap2_gb300.gpu import Model
+    region, nd = sy.region_64x64(size=9), 1460
+    P, T, S = sy.forcing(region, nd, seed=4)
+    launches = []
+    for kd in (1, 4):
+        m = Model(region, max_days=nd, days_per_step=kd, precision="fp32", members=members)
+        m.upload_forcing(0, P, T, S)
+        m.chunk_steps(16 // kd)
+        before = m.launch_count
+        m.run_days(1, 0, nd)
+        m.synchronize()
+        launches.append(m.launch_count - before)
+    assert launches[0] == launches[1]

@@ -392,10 +392,10 @@ bool valid_block_threads(int threads, int precision, int members) {
 }
 
 // An ensemble's states for every thread that the GPU holds of its wavefront.
-size_t states_per_thread(const wg_ctx *ctx) {
+double states_per_thread(const wg_ctx *ctx) {
   int nsm = 0;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
-  return ctx->members > 1 && nsm > 0 ? ctx->nstate() / ((size_t)nsm * PipeBounds<float, true>::threads) : 0;
+  return ctx->members > 1 && nsm > 0 ? (double)ctx->nstate() / ((double)nsm * PipeBounds<float, true>::threads) : 0.;
 }
 
 // An ensemble's launches for the context's block size. Wavefront: blocks are joined up to
@@ -409,7 +409,7 @@ size_t states_per_thread(const wg_ctx *ctx) {
 void set_ensemble_shape(wg_ctx *ctx) {
   constexpr int kMost = PipeBounds<float, true>::threads;
   ctx->layout.join = kMost / ctx->threads;
-  if (states_per_thread(ctx) < 1 ||
+  if (ctx->thread_states < 1 ||
       ctx->blocks_fused / ctx->layout.join != pipeline_max_blocks<float>(true, true, ctx->threads * ctx->layout.join))
     ctx->layout.join = 1;
   ctx->threads_va = std::min(ctx->threads, 64);
@@ -1181,6 +1181,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
   if (cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->upload_done, cudaEventDisableTiming) != cudaSuccess)
     return WG_ERR_CUDA;
+  ctx->thread_states = states_per_thread(ctx.get());
   std::vector<uint32_t> cls(n);
   for (int i = 0; i < n; ++i) cls[i] = work_class(r, i);
   if (!opt->block_threads && ctx->members == 1) ctx->layout = default_layout(ctx.get());
@@ -1203,7 +1204,7 @@ wg_status wg_create(const wg_region *r, const wg_options *opt, wg_ctx **out) {
       if (ctx->glwd.unit_of[i] >= 0) node_of[i] = first[ctx->glwd.unit_of[i]];
   }
   wg_status st = build_topology(n, r->downstream, r->rout_order, cls.data(), &ctx->layout, ctx->topo,
-                                aggr ? node_of.data() : nullptr, states_per_thread(ctx.get()) >= 1);
+                                aggr ? node_of.data() : nullptr, ctx->thread_states >= 1);
   if (st != WG_OK) {
     if (aggr && st == WG_ERR_TOPOLOGY)
       t_create_err = "GLWD units: the cells of a unit drain out of it and back in (no wavefront order)";
@@ -1919,7 +1920,7 @@ struct StepSync { DevSync sync; double *outq; DevWaterTemp wt; };
 static StepSync step_sync(wg_ctx *ctx, int kd, bool one_step = false) {
   StepSync r{ctx->sync, ctx->outq, ctx->wt};
   r.sync.rows = 2;
-  r.sync.data = ctx->outq_days > 0 && !ctx->sync.flow && !ctx->cells_skipped() && !one_step;
+  r.sync.data = ctx->waits() && !one_step;
   r.sync.keep_from = INT_MAX;
   if (r.sync.data) {
     const size_t skip = (size_t)2 * ctx->days_per_step * ctx->nstate();
@@ -2025,7 +2026,7 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
       e = launch_vertical_ahead(c, s, ctx->forcing, ctx->mem, ctx->balance, ring, doy0, fday0, ndays, a, va_end,
                                 ctx->members > 1 ? ctx->blocks_va_alone : ctx->blocks_fused,
                                 ctx->members > 1 ? ctx->threads_va : ctx->threads, ctx->stream, ctx->mon, oday0,
-                                states_per_thread(ctx) >= 8);
+                                ctx->thread_states >= 8);
       ctx->launches++;
     }
     if (ev) cudaEventRecord(ev[1], ctx->stream);

@@ -107,6 +107,7 @@ struct wg_ctx {
   std::vector<char> host_rows;             // a small state on its way to the caller's arrays
   uint8_t *d_active = nullptr;             // wg_set_active_cells (slot order)
   int staging_days = 0;
+  double thread_states = 0.;                 // an ensemble's states for every thread the GPU holds of its wavefront
   int64_t launches = 0;
   std::vector<void *> allocs;
   std::string err;
@@ -212,21 +213,30 @@ struct wg_ctx {
   // wavefront steps of a run of ndays days, kd days per step
   int total_steps(int ndays, int kd) const { return (ndays + kd - 1) / kd + topo.nlevel - 1; }
   int total_steps(int ndays) const { return total_steps(ndays, days_per_step); }
+  // the steps of a call wait for the upstream outflows themselves (else at a grid barrier
+  // or for step flags)
+  bool waits() const { return outq_days > 0 && !sync.flow && !cells_skipped(); }
   // Days per step of a run made in one call (wg_run_days, the deferred per-day
   // calls): at most days_per_step, and fewer where the run is short against the
   // drainage depth.  A step takes the time of one cell's days, one after the other
-  // (t each), and a fixed part (its barrier and the loads it starts with: fixed x
-  // t), so a run costs (ceil(D / kd) + levels - 1) (fixed + kd) t beside its
-  // throughput: with kd days per step the fill and drain of levels - 1 steps last
-  // kd days each.  fixed was measured from runs at 1, 2, 3 and 5 days per step:
-  // 0.25 for one member (65,000 to 550,000 cells, FP64 and FP32), 6 for ensembles,
-  // whose steps start with more loads and whose days overlap across members.
-  // Global grid, one year (198 levels), 1 / 2 / 5 days per step: 18.6 / 21.4 /
-  // 30.6 ms, with water temperature, half a year: 22.0 / 30.2 / 51.2 ms, 550,000
-  // cells in FP32, 90 days: 11.0 / 13.3 / 21.6 ms, 64 FP32 members, 90 days: 33.7
-  // / 31.3 / 36.7 ms (this rule: 1, 1, 1 and 2).  Results do not depend on it.
+  // (t each), and a fixed part (its barrier, the loads it starts with, an ensemble's
+  // groups of states that have no day in it: fixed x t), so a run costs
+  // (ceil(D / kd) + levels - 1) (fixed + kd) t beside its throughput: with kd days per
+  // step the fill and drain of levels - 1 steps last kd days each.  fixed, fitted to
+  // whole runs at 1 to 10 days per step (ms; the first figure is the rule's where no
+  // other is named):
+  // - one member waiting for outflows: 0, one day is the best step at every length (64 x
+  //   64 region, 1,460 days 11.9 / 13.1 at 2; 9,000 cells, 1,000 days 17.4 / 19.6; FP32
+  //   11.8 / 13.3; global grid, one year 14.3 / 17.3).  With 0.25 the first three took 2.
+  // - one member at a barrier: 0.25 (64 x 64 region 15.3 / 15.5; 9,000 cells 23.2 / 21.7:
+  //   the rule takes 2; FP32 16.5 / 14.5: 2).
+  // - ensembles: half the states for each thread that the GPU holds, since every warp
+  //   passes over all of its states in every step: 9,000 x 33, 40 days 1.8 / 2.2 at 2;
+  //   67,420 x 12, 90 days 6.9 / 7.5; x 64 26.2 / 23.3 / 22.9 / 24.0 at 1, 2, 3, 5 (the
+  //   rule: 3); x 128 53.1 / 45.6 / 44.0 / 43.6 (3); x 256 104 / 89 / 86 / 85 (5).
+  // Results do not depend on it.
   int run_days_per_step(int ndays) const {
-    const double fixed = members > 1 ? 6.0 : 0.25;
+    const double fixed = members > 1 ? 0.5 * thread_states : waits() ? 0. : 0.25;
     int best = 1;
     for (int kd = 2; kd <= days_per_step; ++kd)
       if (total_steps(ndays, kd) * (fixed + kd) < total_steps(ndays, best) * (fixed + best)) best = kd;
