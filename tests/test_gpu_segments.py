@@ -167,3 +167,15 @@ def test_a_mask_set_in_mid_run(temp):
         m.run_steps(DOY0, 0, ND, 80, total)
         got.append(_all(m, temp))
     _same(*got)
+
+
+@pytest.mark.parametrize("mask,what", [(False, "upstream outflow"), (True, "grid barrier")])
+def test_a_wait_that_runs_out_says_which(mask, what):
+    from watergap2_gb300.gpu import WgError
+    m = _model()
+    if mask:
+        m.set_active_cells(np.ones(m.region.ncell))
+    m.barrier_test(1)
+    m.run_steps(DOY0, 0, ND, 0, 10)
+    with pytest.raises(WgError, match=what):
+        m.synchronize()

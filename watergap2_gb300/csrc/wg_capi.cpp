@@ -2148,7 +2148,8 @@ wg_status wg_synchronize(wg_ctx *ctx) {
   e = cudaMemcpy(&flag, ctx->sync.error, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "synchronize");
   if (flag) {
-    ctx->err = "grid barrier wait exceeded its iteration limit";
+    ctx->err = flag == 2 ? "wait for an upstream outflow exceeded its iteration limit"
+                         : "grid barrier or step flag wait exceeded its iteration limit";
     return WG_ERR_TIMEOUT;
   }
   return WG_OK;

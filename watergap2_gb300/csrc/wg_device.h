@@ -291,7 +291,7 @@ constexpr unsigned long long kNoOutflow = ~0ull;
 
 struct DevSync {
   unsigned int *counter;   // monotonic arrival counter of the grid barrier
-  int *error;              // 0 ok, nonzero: a barrier wait exceeded its limit (WG_ERR_TIMEOUT)
+  int *error;              // 0 ok; a wait exceeded its limit (WG_ERR_TIMEOUT): 1 barrier or step flag, 2 outflow
   // step flags of the single-member layout (flow != 0): instead of a grid barrier
   // per step, each warp of cells publishes the last step it completed (relative
   // to the launch's first step, -1 before it) and waits only for the warps that

@@ -125,7 +125,7 @@ __device__ __forceinline__ bool has_outflow(const DevSync &sync, const double *p
 // or elsewhere in the grid.
 __device__ __forceinline__ bool wait_ran_out(const DevSync &sync, unsigned &it) {
   if (++it <= WG_DATA_SPIN_LIMIT && ((it & 255u) != 0u || !*(volatile int *)sync.error)) return false;
-  atomicExch(sync.error, 1);
+  atomicExch(sync.error, 2);
   return true;
 }
 
