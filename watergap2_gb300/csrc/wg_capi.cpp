@@ -1916,16 +1916,13 @@ wg_status wg_step_routing(wg_ctx *ctx, int32_t doy, int32_t oday) {
 // the two rows of the barrier whatever the calls wait for, so that a call may follow
 // any other (a graph captured earlier, one under another mask or wg_set_step_sync, the
 // same steps again); the rows of the waits hold nothing from one call to the next.
-struct StepSync { DevSync sync; double *outq; DevWaterTemp wt; };
+struct StepSync { DevSync sync; double *outq; DevWaterTemp wt; int keep_from; };
 static StepSync step_sync(wg_ctx *ctx, int kd, bool one_step = false) {
-  StepSync r{ctx->sync, ctx->outq, ctx->wt};
+  StepSync r{ctx->sync, ctx->outq, ctx->wt, INT_MAX};
   r.sync.rows = 2;
   r.sync.data = ctx->waits() && !one_step;
-  r.sync.keep_from = INT_MAX;
   if (r.sync.data) {
     const size_t skip = (size_t)2 * ctx->days_per_step * ctx->nstate();
-    r.sync.kept = r.outq;
-    r.sync.kept_t = r.wt.outt;
     r.outq += skip;
     if (r.wt.outt) r.wt.outt += skip;
     r.sync.rows = ctx->outq_days / kd;
@@ -1934,17 +1931,28 @@ static StepSync step_sync(wg_ctx *ctx, int kd, bool one_step = false) {
 }
 
 // The two rows at a call of steps [t_b, t_e): what the step before left goes to the row
-// that step t_b reads, and the launches write them from keep_from on. Each step
-// overwrites its parity's row, so that takes the call's last two steps and those from
-// which on the first cells are done with the run. A whole run leaves them as they are.
-// (A call of one step waits for nothing and works in the two rows themselves.)
-static cudaError_t kept_rows(wg_ctx *ctx, StepSync &ss, int kd, int ndays, int t_b, int t_e) {
+// that step t_b reads, and the rows of the waits from step keep_from on go to them,
+// before a launch overwrites those and at the end (keep_outflow).  Each step overwrites
+// its parity's row, so that takes the call's last two steps and those from which on the
+// first cells are done with the run. A whole run leaves the two rows as they are, and a
+// call of one step waits for nothing and works in them. (Steps that wrote both rows
+// themselves cost every run 0.3 %; reading the two rows in the first step would be a
+// race, since a cell two steps ahead overwrites what the one below it needs.)
+static cudaError_t fetch_outflow(wg_ctx *ctx, StepSync &ss, int kd, int ndays, int t_b, int t_e) {
   if (!ss.sync.data || (t_b == 0 && t_e == ctx->total_steps(ndays, kd))) return cudaSuccess;
-  ss.sync.keep_from = std::min(t_e - 2, (ndays + kd - 1) / kd - 3);
+  ss.keep_from = std::max(t_b, std::min(t_e - 2, (ndays + kd - 1) / kd - 3));
   if (t_b == 0) return cudaSuccess;
   const size_t row = (size_t)kd * ctx->nstate(), to = (t_b - 1) % ss.sync.rows * row, from = ((t_b - 1) & 1) * row;
-  return launch_fetch_row(ss.outq + to, ss.sync.kept + from, ss.wt.enabled ? ss.wt.outt + to : nullptr,
-                          ss.wt.enabled ? ss.sync.kept_t + from : nullptr, row, ctx->stream);
+  return launch_fetch_row(ss.outq + to, ctx->outq + from, ss.wt.enabled ? ss.wt.outt + to : nullptr,
+                          ss.wt.enabled ? ctx->wt.outt + from : nullptr, row, ctx->stream);
+}
+// the steps up to a, before a launch that writes rows up to step b - 1's
+static cudaError_t keep_outflow(wg_ctx *ctx, StepSync &ss, const int32_t *offset, int kd, int ndays, int a, int b) {
+  if (ss.keep_from >= a || ss.keep_from > b - 1 - ss.sync.rows) return cudaSuccess;
+  const int from = ss.keep_from;
+  ss.keep_from = a;
+  return launch_keep_outflow(ss.outq, ss.wt.enabled ? ss.wt.outt : nullptr, ctx->outq, ctx->wt.outt, offset, ctx->n, kd,
+                             ss.sync.rows, ndays, from, a, ctx->stream);
 }
 
 // Steps [t_b, t_e) of the day-pipelined wavefront of a run of ndays days, in
@@ -1961,7 +1969,7 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
   ring.days_per_step = kd;
   const bool ov = ctx->overlap();
   StepSync ss = step_sync(ctx, kd, t_e - t_b == 1);
-  const cudaError_t ke = kept_rows(ctx, ss, kd, ndays, t_b, t_e);
+  const cudaError_t ke = fetch_outflow(ctx, ss, kd, ndays, t_b, t_e);
   if (ke != cudaSuccess) return cuda_fail(ctx, ke, "run_steps");
   // (waiting for outflows, a launch's steps have rows of their own beside the one before)
   const int chunk = ss.sync.data ? std::min(ctx->eff_chunk(kd), ss.sync.rows - 1) : ctx->eff_chunk(kd);
@@ -2034,6 +2042,7 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
     vw.t_e = std::min(t_e, b + chunk);
     vw.warps = (ov && vw.t_e > vw.t_b) ? ctx->layout.va_warps : 0;
     vw.nitems = (ov && vw.t_e > vw.t_b) ? (int)((ctx->nstate() + 31) / 32) : 0;
+    if (e == cudaSuccess) e = keep_outflow(ctx, ss, c.offset, kd, ndays, a, b);
     if (e == cudaSuccess)
       e = launch_pipeline(true, c, s, v, ctx->forcing, ctx->mem, ctx->balance, ring, ss.sync, ss.outq, ctx->qst,
                           doy0, fday0, oday0, ndays, a, b, ctx->blocks_fused, ctx->threads, ctx->layout, ctx->mon,
@@ -2042,7 +2051,7 @@ static wg_status run_steps_impl(wg_ctx *ctx, const DevCellsT<R> &c, const DevSta
     if (ev) cudaEventRecord(ev[2], ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "run_steps");
   }
-  return WG_OK;
+  return cuda_fail(ctx, keep_outflow(ctx, ss, c.offset, kd, ndays, t_e, INT_MAX), "run_steps");
 }
 
 extern "C" {

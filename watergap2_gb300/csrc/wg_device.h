@@ -304,11 +304,6 @@ struct DevSync {
   // cell's outflow of the step before waits until the value is there, and there is
   // no barrier between steps.  rows: the buffer's rows, step t in row t % rows
   int32_t rows, data;
-  // (data) a run's outflows between calls: two rows, step t in row t & 1, of the outflow
-  // and of the river temperature, which steps from keep_from on write too (no step
-  // reads them: a cell two steps ahead of one below it would overwrite what that needs)
-  double *kept, *kept_t;
-  int32_t keep_from;
   // failure-detection test: arrivals the grid barrier waits for beyond the grid's
   // blocks, and with data nonzero values not taken for outflow (0 in every run; 1
   // makes each wait run out, see wg_set_barrier_test)

@@ -788,15 +788,11 @@ __global__ void __launch_bounds__(WaveBounds<R, ENS, VAW>::threads, WaveBounds<R
           }
           if (ENS) q_now[si] = (double)tv;
           else st_outflow(q_now + si, (double)tv);
-          const bool keep = FUSED && !ENS && t >= sync.keep_from;
-          const size_t kept_at = ((size_t)(t & 1) * kd + kk) * N + si;
-          if (keep) st_outflow(sync.kept + kept_at, (double)tv);
           if constexpr (WT) {
             // a cell without continental area keeps the reference's initial 15 degrees (routing.cpp:174)
             const double tr = nocont ? 15. : wtd.river((double)rs.river, (double)c.rlen[s], (double)c.cfa[s],
                                                        (double)o.owpet);
             st_outflow(t_now0 + (size_t)kk * N + si, tr);
-            if (keep) st_outflow(sync.kept_t + kept_at, tr);
             const int stw = c.station[s];
             if (stw >= 0) wtp.qst_t[(size_t)(oday0 + d) * c.nstation + stw] = tr;
           }
@@ -1125,6 +1121,30 @@ __global__ void __launch_bounds__(256) k_fetch_row(double *dst, const double *sr
 cudaError_t launch_fetch_row(double *dst, const double *src, double *dst_t, const double *src_t, size_t n, cudaStream_t st) {
   const dim3 grid((unsigned)std::min<size_t>((n + 255) / 256, 152 * 32), dst_t ? 2 : 1);
   k_fetch_row<<<grid, 256, 0, st>>>(dst, src, dst_t, src_t, n);
+  return cudaGetLastError();
+}
+
+// What a wavefront of two rows (one member, a grid barrier per step) holds of steps [a,
+// b): per cell and day of the step the last two steps that had such a day.
+__global__ void __launch_bounds__(256) k_keep_outflow(const double *rows, const double *rows_t, double *kept, double *kept_t,
+                                                      const int32_t *__restrict__ offset, int n, int kd, int nrows,
+                                                      int ndays, int a, int b) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, row = (size_t)kd * n;
+  if (i >= row) return;
+  const int s = (int)(i % n), left = ndays - 1 - (int)(i / n);   // from this place in the first step to the last day
+  if (left < 0) return;
+  const int first = max(a, offset[s]), last = min(b - 1, offset[s] + left / kd);
+  for (int t = max(first, last - 1); t <= last; ++t) {
+    kept[(t & 1) * row + i] = rows[t % nrows * row + i];
+    if (rows_t) kept_t[(t & 1) * row + i] = rows_t[t % nrows * row + i];
+  }
+}
+
+cudaError_t launch_keep_outflow(const double *rows, const double *rows_t, double *kept, double *kept_t,
+                                const int32_t *offset, int n, int kd, int nrows, int ndays, int a, int b,
+                                cudaStream_t st) {
+  k_keep_outflow<<<(unsigned)(((size_t)kd * n + 255) / 256), 256, 0, st>>>(rows, rows_t, kept, kept_t, offset, n, kd,
+                                                                          nrows, ndays, a, b);
   return cudaGetLastError();
 }
 

@@ -81,6 +81,12 @@ cudaError_t launch_fill(double *p, size_t n, double v, cudaStream_t st);
 // out, in nrows rows of n cells x members
 cudaError_t launch_clear_skipped(double *rows, double *rows_t, const uint8_t *active, int n, int members, int nrows,
                                  cudaStream_t st);
+// the outflow rows of steps [a, b) (step t in row t % nrows) into the two rows kept
+// between calls (step t in row t & 1), each cell's last steps of either parity; the river
+// temperature's likewise (null: none)
+cudaError_t launch_keep_outflow(const double *rows, const double *rows_t, double *kept, double *kept_t,
+                                const int32_t *offset, int n, int kd, int nrows, int ndays, int a, int b,
+                                cudaStream_t st);
 // n doubles from src to dst and, where there are any, from src_t to dst_t
 cudaError_t launch_fetch_row(double *dst, const double *src, double *dst_t, const double *src_t, size_t n, cudaStream_t st);
 template <class R>
