@@ -35,7 +35,7 @@ sys.path.insert(0, ROOT)
 METRIC = "cell-days/s on 1 GB300 (plain FP64 vs batched FP32 ensemble) at stated error"
 DAYS_PER_STEP = 365
 # days every cell advances per wavefront step (wg_options.days_per_step): the
-# step barrier and the start-of-step load latency are paid once per 5 days; a
+# wait for upstream outflows and the start-of-step load latency are paid once per 5 days; a
 # timed step (one year) is 73 wavefront steps.  Results are the same bits.
 WAVEFRONT_DAYS = 5
 WSTEPS_PER_YEAR = DAYS_PER_STEP // WAVEFRONT_DAYS

@@ -541,8 +541,9 @@ wg_status wg_save_snapshot(wg_ctx *ctx);
 wg_status wg_restore_snapshot(wg_ctx *ctx);
 
 /* Kernel timing: with enable != 0, wg_run_steps records CUDA events on the
- * context's stream around each launch of the vertical-ahead kernel and of the
- * wavefront kernel; wg_get_kernel_times synchronises and returns the summed
+ * context's stream around each launch of the vertical-ahead kernel (with the pass
+ * before it that computes the potential evapotranspiration) and of the wavefront
+ * kernel (with the copies of outflow rows before it); wg_get_kernel_times synchronises and returns the summed
  * device time of each since the last call (or since enabling), and the number
  * of launch pairs.  Launches inside a captured graph are not timed. */
 wg_status wg_kernel_timing(wg_ctx *ctx, int32_t enable);
@@ -621,9 +622,10 @@ wg_status wg_measure_fp64_peak(int32_t device, double *tflops);
  * read for fn 2 only. */
 wg_status wg_math_eval(int32_t device, int32_t fn, const double *x, const double *y, int64_t n, double *out);
 
-/* Information: number of drainage levels (longest flow path + 1), kernel
- * launches issued so far (the passes over the forcing that prepare a run are not
- * counted), and the last CUDA error string. */
+/* Information: number of drainage levels (longest flow path + 1), kernel launches
+ * issued so far (uploads, vertical balance, wavefront, balance sums; not counted: the
+ * pass over the forcing that computes a run's potential evapotranspiration, copies of
+ * outflow rows, reads put into cell order), and the last CUDA error string. */
 int32_t wg_num_levels(const wg_ctx *ctx);
 int64_t wg_launch_count(const wg_ctx *ctx);
 /* wg_last_error(NULL): why the calling thread's last wg_create failed. */

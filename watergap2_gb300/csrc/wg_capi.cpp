@@ -602,7 +602,6 @@ wg_status alloc_state(wg_ctx *ctx, DevStateT<R> &s, DevVertT<R> &v) {
   return v.land_leak ? WG_OK : WG_ERR_NOMEM;
 }
 
-// Copy one member's state between host arrays (cell order, double) and the device.
 // Device memory into the caller's arrays, after the work on the context's stream: in
 // one piece through a kept host buffer where that is all (the copies lie in the
 // staging in order), else one by one into pages that have been touched -- the copy
@@ -634,7 +633,8 @@ cudaError_t copy_out(wg_ctx *ctx, const HostCopy *copies, size_t count) {
 // FP32 values into doubles) on the device, as many as the staging holds at a time,
 // and copied from there -- a small state in one copy, larger fields straight into
 // the caller's arrays.  One strided copy and one scatter loop per field on the host
-// took 3.0 ms for 67,420 cells and 30 ms for 550,000; this takes 0.63 and 3.0 ms.
+// took 3.0 ms for 67,420 cells and 30 ms for 550,000; this takes 0.63 and, into arrays
+// fresh from the allocator, 3.0 to 4.1 ms.
 template <class R>
 wg_status read_state(wg_ctx *ctx, const DevStateT<R> &s, const wg_state_view *v, int member) {
   const size_t n = ctx->n, N = ctx->nstate();
@@ -695,6 +695,7 @@ bool rows_to_host(wg_ctx *ctx, const double *src, size_t rows, double *out, cuda
   return true;
 }
 
+// Copy one member's state between host arrays (cell order, double) and the device.
 template <class R>
 wg_status copy_state(wg_ctx *ctx, const DevStateT<R> &s, const wg_state_view *v, int member, bool to_device) {
   if (!to_device && read_state_fits(ctx)) return read_state(ctx, s, v, member);

@@ -8,10 +8,11 @@
 //                  day d at step d + offset(n), offset = longest flow path -
 //                  distance of n to its outlet.  Every upstream cell of n then
 //                  has offset(n) - 1 and delivers day d's outflow exactly one step
-//                  earlier.  A cell waits for these outflows themselves (one FP64
-//                  member; rows of the outflow buffer per step), or all cells for
-//                  a grid barrier per step (ensembles, GLWD units, runs with
-//                  skipped cells) or, optionally, for per-warp step flags.  Cells
+//                  earlier.  A cell waits for these outflows themselves (one
+//                  member, FP64 or FP32; rows of the outflow buffer per step), or
+//                  all cells for a grid barrier per step (ensembles, GLWD units,
+//                  runs with skipped cells) or, optionally, for per-warp step
+//                  flags.  Cells
 //                  without a water body take their vertical balance from the ring
 //                  that k_vertical_ahead filled; the monthly output aggregates are
 //                  accumulated in its epilogue.  With ENS the cells carry
@@ -28,6 +29,8 @@
 //                  a chunk of days, state in registers, into the ring.
 //  k_state_rows / k_rows   state, output grids, water use and water temperature
 //                  into cell order for reading.
+//  k_fetch_row / k_keep_outflow / k_clear_skipped   the outflow rows that lie
+//                  between the calls of a run.
 //  k_math_eval     the FP64 path's exp/log/pow/reciprocal on arrays (tests).
 //  k_unf_forcing / k_gather_forcing  forcing uploads into the slot layout.
 //  k_volume / k_balance_sum   compensated (Neumaier) FP64 water-balance sums.
