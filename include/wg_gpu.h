@@ -567,7 +567,7 @@ int32_t wg_get_chunk_steps(const wg_ctx *ctx);
  * FP64 pipe has that work while the routing warps wait; the first chunk of each
  * call runs its vertical balance in a launch of its own.  On by default where
  * the shape allows it.  enable = 0 switches it off (one vertical-ahead launch
- * before each wavefront launch); WG_ERR_UNSUPPORTED where the shape has no room
+ * before each chunk's wavefront launches); WG_ERR_UNSUPPORTED where the shape has no room
  * for it.  wg_get_vertical_overlap returns the extra warps per block, at least 1
  * (0: off).  Results are the same bits either way. */
 wg_status wg_set_vertical_overlap(wg_ctx *ctx, int32_t enable);
